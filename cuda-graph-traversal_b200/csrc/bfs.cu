@@ -44,8 +44,13 @@
 namespace g5 {
 
 constexpr int BFS_THREADS = 256;
-constexpr unsigned BFS_CHUNK = 256;  // default: edges of a long row taken by one warp
-constexpr unsigned BFS_BIG_DEG = BIG_DEG;  // default: longest row expanded by one warp
+// Defaults: edges of a long row taken by one warp, and the longest row a warp
+// expands by itself.  A warp step of 32 edges is a chain of a few dependent
+// round trips, so the two bound a short level: on 700 K vertices (a level of
+// 36 rows with 64 K edges) 128 / 256 takes 95 us, 256 / 256 103 and 256 /
+// 1024 139; on 34 M vertices 732, 742 and 758.
+constexpr unsigned BFS_CHUNK = 128;
+constexpr unsigned BFS_BIG_DEG = 256;
 constexpr unsigned BFS_STAGE = 512;  // per-warp staging of the next queue (16 KiB shared per block)
 constexpr unsigned long long SOLO_EDGES = 4096;  // levels at most this wide run in block 0 alone
 constexpr int BFS_TRACE = 64;                    // levels recorded in the control block
@@ -63,8 +68,11 @@ static_assert(sizeof(LevelState) % 8 == 0, "LevelState is copied in 8-byte words
 struct BfsCtl {
     g5_bfs_stats res;     // the search's result (same layout as the C ABI's)
     const uint32_t *init_used;  // visited bitmap the last reset started from (nullptr: all clear)
-    unsigned bar;         // grid barrier arrivals
-    unsigned n_small[3];  // per level slot: queue entries of degree <= BIG_DEG
+    // Words that waiting blocks poll have lines of their own, apart from the
+    // counters that working blocks add to (sharing one, 592 blocks took 95 us
+    // for 4 K vertices instead of 71, and 134 for 700 K instead of 124).
+    alignas(128) unsigned bar;  // grid barrier arrivals
+    alignas(128) unsigned n_small[3];  // per level slot: queue entries of degree <= BIG_DEG
     unsigned long long big[3];  //           big entries << 40 | their chunks
     unsigned grab[3];     //                 work cursor over the small part
     unsigned cgrab[3];    //                 work cursor over the big part's chunks
@@ -72,9 +80,9 @@ struct BfsCtl {
     unsigned ulen[3];     //                 bottom-up: entries of the unvisited list
     unsigned long long m_next[3];  //        degree sum of the next frontier
     // hand-off from the solo prologue to the grid
-    unsigned long long go;  // launch sequence << 2 | 1 (continue on the grid) or 2 (finished)
+    alignas(128) unsigned long long go;  // launch sequence << 2 | 1 (continue on the grid) or 2 (finished)
     unsigned heartbeat;     // solo levels completed so far (waiters restart their clock on change)
-    unsigned hand_fb;  // 1 when the frontier bitmap is the second buffer
+    alignas(128) unsigned hand_fb;  // 1 when the frontier bitmap is the second buffer
     LevelState hand;
     // per-level trace: time at the level's end, frontier size and edges, direction
     unsigned long long t0;
@@ -179,7 +187,7 @@ __device__ __forceinline__ void td_visit(const BfsArgs &a, const WarpStage &bq, 
         atomicOr(&a.ctl->res.error_flags, DEVERR_CAPACITY);
 }
 
-__device__ void td_expand(const BfsArgs &a, const WarpStage &bq, int level, int cur, int s_cur, int s_nxt,
+__device__ void td_expand(const BfsArgs &a, const WarpStage &bq, int level, int cur, int s_cur, int s_nxt, bool solo,
                           unsigned long long &my_m) {
     BfsCtl *c = a.ctl;
     const unsigned lane = lane_id();
@@ -191,13 +199,16 @@ __device__ void td_expand(const BfsArgs &a, const WarpStage &bq, int level, int 
     const unsigned long long bp = ld_volatile(&c->big[s_cur]);
 
     // Small part: g queue entries per grab, edges gathered across the warp.
-    const unsigned g = grab_size(ns, ((unsigned long long)gridDim.x * blockDim.x) >> 5);
-    for (;;) {
-        unsigned base = 0;
-        if (lane == 0) base = atomicAdd(&c->grab[s_cur], g);
-        base = __shfl_sync(FULL, base, 0);
-        if (base >= ns) break;
-        const unsigned i = base + lane;
+    // Each warp's first grab (and chunk, below) is its own number's, the rest
+    // come from the counter: an atomic per warp on one word, 4736 of them
+    // even for an empty list, took longer than a short level's work.
+    // Neighbouring grabs go to different SMs, so that a short list spreads.
+    // (A solo level of block 0 counts its own warps alone.)
+    const unsigned nw = solo ? blockDim.x >> 5 : gridDim.x * (blockDim.x >> 5);
+    const unsigned wg = solo ? threadIdx.x >> 5 : (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    const unsigned g = grab_size(ns, nw);
+    for (unsigned long long base = (unsigned long long)wg * g; base < ns;) {
+        const unsigned long long i = base + lane;
         const bool valid = lane < g && i < ns;
         const unsigned u = valid ? __ldcg(&Q[i]) : 0u;
         const uint64_t rb = valid ? __ldg(&a.rowptr[u]) : 0;
@@ -215,15 +226,14 @@ __device__ void td_expand(const BfsArgs &a, const WarpStage &bq, int level, int 
             const unsigned v = has ? (unsigned)__ldg(&a.col[rbj + (e - exj)]) : 0u;
             td_visit(a, bq, has, v, uj, level + 1, QN, BN, &c->n_small[s_nxt], &c->big[s_nxt], my_m);
         }
+        unsigned b = 0;
+        if (lane == 0) b = atomicAdd(&c->grab[s_cur], g);
+        base = (unsigned long long)nw * g + __shfl_sync(FULL, b, 0);
     }
     // Big part: chunks of every big vertex from one grid-wide counter.
     const unsigned nb = big_count(bp);
     const unsigned long long nch = big_chunks(bp);
-    for (;;) {
-        unsigned ch = 0;
-        if (lane == 0) ch = atomicAdd(&c->cgrab[s_cur], 1u);
-        ch = __shfl_sync(FULL, ch, 0);
-        if (ch >= nch) break;
+    for (unsigned ch = wg; ch < nch;) {
         const unsigned j = chunk_owner(B, nb, ch);
         const unsigned u = __ldcg(&Q[a.n - 1 - j]);
         const uint64_t rb = __ldg(&a.rowptr[u]);
@@ -235,6 +245,9 @@ __device__ void td_expand(const BfsArgs &a, const WarpStage &bq, int level, int 
             const unsigned v = has ? (unsigned)__ldg(&a.col[rb + e]) : 0u;
             td_visit(a, bq, has, v, u, level + 1, QN, BN, &c->n_small[s_nxt], &c->big[s_nxt], my_m);
         }
+        unsigned b = 0;
+        if (lane == 0) b = atomicAdd(&c->cgrab[s_cur], 1u);
+        ch = nw + __shfl_sync(FULL, b, 0);
     }
     if (!stage_flush_warp(bq, QN, a.n, &c->n_small[s_nxt])) atomicOr(&c->res.error_flags, DEVERR_CAPACITY);
 }
@@ -450,10 +463,11 @@ __device__ __forceinline__ int bfs_decide(const BfsArgs &a, int mode, unsigned n
 enum { PEND_NONE = 0, PEND_TO_BITS = 1, PEND_TO_QUEUE = 2 };
 
 // Expands level st.level; adds the next frontier's degree sum and (bottom-up)
-// size into slot s_nxt.  No synchronisation.
+// size into slot s_nxt.  Synchronises the block, not the grid.
 __device__ __forceinline__ void bfs_expand_level(const BfsArgs &a, const WarpStage &bq, const LevelState &st,
-                                                 const unsigned *fb, unsigned *nb, unsigned *zb) {
+                                                 const unsigned *fb, unsigned *nb, unsigned *zb, bool solo) {
     BfsCtl *c = a.ctl;
+    __shared__ unsigned long long s_sum[2];
     const int s_cur = st.level % 3, s_nxt = (st.level + 1) % 3, s_clr = (st.level + 2) % 3;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         c->n_small[s_clr] = 0;
@@ -464,17 +478,25 @@ __device__ __forceinline__ void bfs_expand_level(const BfsArgs &a, const WarpSta
         c->ulen[s_clr] = 0;
         c->m_next[s_clr] = 0;
     }
+    if (threadIdx.x < 2) s_sum[threadIdx.x] = 0;
+    __syncthreads();
     unsigned long long my_m = 0;
     unsigned my_found = 0;
     if (st.mode == TOP_DOWN)
-        td_expand(a, bq, st.level, st.cur, s_cur, s_nxt, my_m);
+        td_expand(a, bq, st.level, st.cur, s_cur, s_nxt, solo, my_m);
     else
         bu_expand(a, bq, st, s_cur, s_nxt, fb, nb, zb, my_m, my_found);
+    // Summed per block: one atomic per block on the level's counters.
     my_m = warp_sum(my_m);
     my_found = warp_sum(my_found);
     if (lane_id() == 0) {
-        if (my_m) atomicAdd(&c->m_next[s_nxt], my_m);
-        if (my_found) atomicAdd(&c->found[s_nxt], my_found);
+        if (my_m) atomicAdd(&s_sum[0], my_m);
+        if (my_found) atomicAdd(&s_sum[1], (unsigned long long)my_found);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (s_sum[0]) atomicAdd(&c->m_next[s_nxt], s_sum[0]);
+        if (s_sum[1]) atomicAdd(&c->found[s_nxt], (unsigned)s_sum[1]);
     }
 }
 
@@ -642,7 +664,7 @@ __global__ void __launch_bounds__(BFS_THREADS, 4) bfs_persistent_kernel(BfsArgs 
         int solo = 0;
         while (a.nblocks == 1 || (st.mode == TOP_DOWN && st.pending == PEND_NONE && st.m_f <= SOLO_EDGES)) {
             if (a.nblocks == 1 && st.pending != PEND_NONE) break;  // conversions run in the grid loop
-            bfs_expand_level(a, bq, st, fb, nb, nullptr);  // top-down only (conversions end the loop)
+            bfs_expand_level(a, bq, st, fb, nb, nullptr, true);  // top-down only (conversions end the loop)
             __threadfence();
             __syncthreads();
             ++solo;
@@ -727,7 +749,7 @@ __global__ void __launch_bounds__(BFS_THREADS, 4) bfs_persistent_kernel(BfsArgs 
             if (!grid_sync(&c->bar, &c->res.error_flags, epoch, a.nblocks, a.limit_ns)) return;
         }
         st.pending = PEND_NONE;
-        bfs_expand_level(a, bq, st, fb, nb, zb);
+        bfs_expand_level(a, bq, st, fb, nb, zb, false);
         if (!grid_sync(&c->bar, &c->res.error_flags, epoch, a.nblocks, a.limit_ns)) return;
         if (!bfs_advance(a, st, fb, nb, zb)) break;
     }
@@ -907,6 +929,17 @@ static BfsWork carve_bfs(void *base, uint64_t n) {
 }
 
 // Largest co-resident grid of the persistent kernel on this device.
+// Blocks of a search by default: one per 256 vertices until each SM has one
+// (a quarter of what fits), from 2^20 vertices on one per 8192.  More blocks
+// than a level has work for only poll the barrier: 4 K vertices take 49 us on
+// 16 blocks, 50 on 148 and 71 on 592; 700 K 95, 97 and 124 on 148, 222 and
+// 592; 2.1 M 226, 175, 173 and 180 on 148, 296, 444 and 592; 34 M 775 on 444
+// and 719 on 592.
+static int bfs_blocks(uint64_t nverts, int max_blocks) {
+    const uint64_t small = std::min<uint64_t>(nverts / 256, (uint64_t)std::max(1, max_blocks / 4));
+    return (int)std::min<uint64_t>(max_blocks, std::max<uint64_t>(1, std::max(small, nverts / 8192)));
+}
+
 static int bfs_max_blocks(int *out) {
     static int cached[64] = {};
     DeviceInfo di;
@@ -1192,8 +1225,7 @@ static int bfs_launch(const BfsWork &w, const uint64_t *d_rowstarts, const int32
     int max_blocks = 0;
     rc = bfs_max_blocks(&max_blocks);
     if (rc) return rc;
-    int blocks = p.blocks > 0 ? std::min(p.blocks, max_blocks)
-                              : (int)std::min<uint64_t>(max_blocks, std::max<uint64_t>(1, nverts / 2048));
+    int blocks = p.blocks > 0 ? std::min(p.blocks, max_blocks) : bfs_blocks(nverts, max_blocks);
     BfsArgs a;
     a.rowptr = d_rowstarts;
     a.col = d_col;
@@ -1767,6 +1799,6 @@ extern "C" int g5_bfs_grid(uint64_t nverts, int32_t *blocks, int32_t *max_blocks
     int rc = bfs_max_blocks(&mb);
     if (rc) return rc;
     *max_blocks = mb;
-    *blocks = (int)std::min<uint64_t>(mb, std::max<uint64_t>(1, nverts / 2048));
+    *blocks = bfs_blocks(nverts, mb);
     return G5_OK;
 }
