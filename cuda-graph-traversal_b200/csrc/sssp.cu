@@ -54,15 +54,15 @@ static_assert(STAGE_R <= 32 && STAGE_Q <= 32, "stage_push writes a full slice wi
 constexpr int SSSP_TRACE = 256;      // phases recorded in the control block
 // List entries with more edges to expand than this go to the big part (cut
 // into SSSP_CHUNK chunks across the grid), and a warp grabs at most SSSP_GRAB
-// small entries at once: a grab holds at most SSSP_GRAB x SSSP_BIG_DEG edges,
+// small entries at once: a grab holds at most SSSP_GRAB times as many edges,
 // so no warp is left with a long tail of relaxations at the end of a phase.
-// Both are defaults of g5_sssp_params.big_deg / .chunk.
-constexpr unsigned SSSP_BIG_DEG = 256;
+// SSSP_CHUNK is the default of both g5_sssp_params.big_deg and .chunk.
 // Chunk of a long row taken by one warp in the frontier, heavy-set and
 // expanded-set lists.  A warp's relaxation steps form a chain of dependent
 // round trips, so the chunk bounds the longest warp of a phase.  A multiple
 // of 32 x SSSP_EDGES (the entries a warp step covers).
-constexpr unsigned SSSP_CHUNK = 256;
+constexpr unsigned SSSP_CHUNK = 128;
+constexpr unsigned SSSP_TILE_SMALL = 64;  // for graphs of up to 2^22 vertices (sssp_tile)
 constexpr unsigned SSSP_GRAB = 32;
 // Sub-buckets: once a bucket's light frontier holds SPLIT_MIN light entries,
 // the rest of the bucket is processed in SUB equal sub-buckets in order
@@ -81,7 +81,16 @@ constexpr unsigned SSSP_GRAB = 32;
 // distance drops several times inside the sub-bucket then re-reads its light
 // row (weights only decide) but repeats none of its random relaxations.
 constexpr int SUB = 32;
-constexpr unsigned long long SPLIT_MIN = 1ull << 25;  // default; g5_sssp_params.sub_min overrides
+// The line: 8.4 M vertices, whose frontier reaches 25 M light entries, take
+// 6.2 ms split from 2^18 to 2^22 on and 7.1 unsplit; 2.1 M vertices, which
+// reach 6 M, 3.0 ms split at 2^20 to 2^22, 3.2 unsplit and 4.6 at 2^18, where
+// the sub-buckets' phases cost more than the repeated relaxations; 600 K,
+// which reach 1.5 M, 2.0 ms unsplit and 2.8 split at 2^20.
+// With many sources (packed graphs) a large frontier is many small ones, whose
+// vertices are seldom lowered again: 90 graphs with 167 M entries in all take
+// 13 ms unsplit and 18 split, so there the line is where it hardly matters.
+// Defaults; g5_sssp_params.sub_min overrides.
+constexpr unsigned long long SPLIT_MIN = 1ull << 22, SPLIT_MIN_MULTI = 1ull << 25;
 constexpr float SSSP_PULL_RATIO = 1.0f;  // default heavy-phase pull threshold
 constexpr double PULL_WALK = 0.25;       // cost of a pull's bitmap walk, in CSR entries per vertex
 constexpr unsigned long long UNREACHED = ~0ull;
@@ -1592,6 +1601,21 @@ static int sssp_max_blocks(int *out) {
     return G5_OK;
 }
 
+// Blocks of a search by default: one per 128 vertices up to the whole device.
+// A phase's rows are spread over all warps, so more blocks shorten it long
+// before there is a vertex per thread (4 K vertices: 2 blocks 777 us, 32 523,
+// 148 517; 16 K: 8 blocks 1165, 148 872; 260 K: 128 blocks 1480, 444 1417).
+static int sssp_blocks(uint64_t nverts, int max_blocks) {
+    return (int)std::min<uint64_t>(max_blocks, std::max<uint64_t>(1, nverts / 128));
+}
+
+// The default of both list tiles.  A warp's steps over a row of 64 edges each
+// are a chain of dependent round trips that bounds a short phase, while on
+// large graphs the lookups of many small chunks cost more than they shorten
+// (64, 128 and 256: 16 K vertices 802, 865 and 915 us, 600 K 1641, 1797 and
+// 2059, 2.1 M 2919, 2948 and 3116, 16.8 M 9610, 8933 and 8972).
+static unsigned sssp_tile(uint64_t nverts) { return nverts <= (1ull << 22) ? SSSP_TILE_SMALL : SSSP_CHUNK; }
+
 }  // namespace g5
 
 using namespace g5;
@@ -1717,8 +1741,7 @@ static int sssp_launch(const uint64_t *d_rowstarts, const int32_t *d_col, const 
     G5_CHECK_ARG((p.perm == nullptr) == (p.inv == nullptr), "%s: give both perm and inv or neither", who);
     int max_blocks = 0;
     if ((rc = sssp_max_blocks(&max_blocks))) return rc;
-    int blocks = p.blocks > 0 ? std::min(p.blocks, max_blocks)
-                              : (int)std::min<uint64_t>(max_blocks, std::max<uint64_t>(1, nverts / 2048));
+    const int blocks = p.blocks > 0 ? std::min(p.blocks, max_blocks) : sssp_blocks(nverts, max_blocks);
     cudaStream_t st = (cudaStream_t)stream;
     SsspArgs a;
     a.rowptr = d_rowstarts;
@@ -1738,7 +1761,7 @@ static int sssp_launch(const uint64_t *d_rowstarts, const int32_t *d_col, const 
     a.nroots = nroots;
     a.delta = p.delta;
     a.pull_ratio = p.pull == 0.0f ? SSSP_PULL_RATIO : p.pull;
-    a.split_min = p.sub_min == 0 ? SPLIT_MIN : p.sub_min < 0 ? ~0ull : (unsigned long long)p.sub_min;
+    a.split_min = p.sub_min == 0 ? (d_roots ? SPLIT_MIN_MULTI : SPLIT_MIN) : p.sub_min < 0 ? ~0ull : (unsigned long long)p.sub_min;
     a.pack = w.pack;
     a.fstamp = w.fstamp;
     a.sstamp = w.sstamp;
@@ -1763,8 +1786,8 @@ static int sssp_launch(const uint64_t *d_rowstarts, const int32_t *d_col, const 
     a.nblocks = (unsigned)blocks;
     a.limit_ns = wait_limit_ns();
     a.check_opens = p.check_opens != 0;
-    a.big_deg = p.big_deg ? (unsigned)p.big_deg : SSSP_BIG_DEG;
-    a.chunk = p.chunk ? (unsigned)p.chunk : SSSP_CHUNK;
+    a.big_deg = p.big_deg ? (unsigned)p.big_deg : sssp_tile(nverts);
+    a.chunk = p.chunk ? (unsigned)p.chunk : sssp_tile(nverts);
     a.perm = p.perm;
     a.inv = p.inv;
     if (p.small && !d_roots) {
@@ -1885,6 +1908,6 @@ extern "C" int g5_sssp_grid(uint64_t nverts, int32_t *blocks, int32_t *max_block
     int rc = sssp_max_blocks(&mb);
     if (rc) return rc;
     *max_blocks = mb;
-    *blocks = (int)std::min<uint64_t>(mb, std::max<uint64_t>(1, nverts / 2048));
+    *blocks = sssp_blocks(nverts, mb);
     return G5_OK;
 }

@@ -407,15 +407,16 @@ int g5_bfs_dist_from_pred(const uint64_t *d_rowstarts, const int32_t *d_col, uin
 
 typedef struct g5_sssp_params {
     float delta;    /* bucket width (default 0.1, the reference's fixed value) */
-    int32_t blocks; /* persistent grid size; 0 = fill the device              */
+    int32_t blocks; /* persistent grid size; 0 = by the graph's size, up to
+                       the whole device                                     */
     float pull;     /* a bucket's heavy phase pulls (each unsettled vertex scans
                        its own heavy entries) when the bucket's rows hold at
                        least pull x the entries of all unsettled vertices'
                        rows; 0 = default (1.0), < 0 = always push           */
     int32_t sub_min; /* once a bucket's light frontier holds this many light
                        CSR entries, the rest of the bucket runs in 32
-                       sub-buckets in distance order; 0 = default (2^25),
-                       < 0 = never                                           */
+                       sub-buckets in distance order; 0 = default (2^22;
+                       2^25 with several sources), < 0 = never                                           */
     int32_t small;   /* 1: the source's component is small (outside the main
                        component): one lean block, label-correcting rounds,
                        same distances and parents; 0 = the bucketed search  */
@@ -429,9 +430,10 @@ typedef struct g5_sssp_params {
                        "held a vertex twice") if a queue held a vertex twice;
                        a test aid, same results; 0 = plain stores (default) */
     int32_t big_deg; /* list entries with more edges to expand are cut into
-                       chunks across the grid; 0 = default (256)            */
+                       chunks across the grid; 0 = by the graph's size (64
+                       up to 2^22 vertices, else 128)                       */
     int32_t chunk;   /* edges per chunk, a multiple of 64 up to 65536; 0 =
-                       default (256).  Neither tile changes a result        */
+                       likewise.  Neither tile changes a result             */
     const uint32_t *perm; /* renumbered search (both set, from
                        g5_csr_sssp_renumber) or not (both NULL): the CSR
                        arguments (row starts, column, weights, light and
