@@ -27,6 +27,9 @@
 //     reference clears N visited flags per light iteration, :270-275).
 //   * a settled bitmap (N/8 bytes, L2 resident): edges into vertices of
 //     finished buckets are skipped without touching their distance.
+//   * once the rows of the vertices not settled yet hold few entries, the
+//     kernel ends and a second one finishes the search as one label-
+//     correcting run (sssp_finish_kernel).
 //   * frontiers are processed with the warp-gather / big-vertex sharing of
 //     the BFS kernel, over the light or the heavy part of each row.
 //
@@ -91,6 +94,19 @@ constexpr int SUB = 32;
 // 13 ms unsplit and 18 split, so there the line is where it hardly matters.
 // Defaults; g5_sssp_params.sub_min overrides.
 constexpr unsigned long long SPLIT_MIN = 1ull << 22, SPLIT_MIN_MULTI = 1ull << 25;
+// The bucketed kernel hands over to sssp_finish_kernel once the rows of the
+// vertices not settled hold at most FINISH_ENTRIES entries or 2^-FINISH_SHIFT
+// of all.  What is left after the bucket that holds the hubs hangs off settled
+// vertices and is seldom lowered twice, but it went through some 20 buckets
+// of at least three phases, about 10 us each however small: with the finish
+// 600 K vertices take 1.1 ms instead of 1.5, 90 packed graphs 8.9 instead of
+// 11.7.  A search handed over at once relaxes each entry about five times,
+// which beats the buckets' phases up to about 2^20 entries (16 K vertices:
+// 0.24 ms, in buckets 0.67).  A kernel of its own because the bucketed one is
+// as large as it should get: with this loop inside, it spilled three times as
+// much.
+constexpr unsigned long long FINISH_ENTRIES = 1ull << 20;
+constexpr int FINISH_SHIFT = 2;
 constexpr float SSSP_PULL_RATIO = 1.0f;  // default heavy-phase pull threshold
 constexpr double PULL_WALK = 0.25;       // cost of a pull's bitmap walk, in CSR entries per vertex
 constexpr unsigned long long UNREACHED = ~0ull;
@@ -166,12 +182,18 @@ struct SsspCtl {
     unsigned dbg_claim;
     unsigned long long dbg[7];
     // per-phase trace: end time, kind (0 open, 1 light, 2 heavy push, 3
-    // heavy pull), input size, edges looked at so far
+    // heavy pull, 4 sub-bucket open, 5 split, 6 settle, 7 finish), input
+    // size, edges looked at so far
     unsigned long long t0;
     unsigned long long t_phase[SSSP_TRACE];
     unsigned long long e_phase[SSSP_TRACE];
     unsigned n_phase[SSSP_TRACE];
     unsigned char kind_phase[SSSP_TRACE];
+    // sssp_finish_kernel: its grid barrier, then per round slot its lists'
+    // sizes (entries << 32 | units) and the cursors over their chunks.
+    alignas(128) unsigned fbar;
+    alignas(128) unsigned long long fin[3];
+    unsigned fgrab[3];
 };
 
 // Output arrays that g5_sssp_reset pre-filled with -1.0f / -1.  When the
@@ -224,6 +246,8 @@ struct SsspArgs {
     bool check_opens;  // opens exchange their stamps and flag a vertex met twice (DEVERR_DUPLICATE)
     unsigned big_deg;  // list entries with more edges to expand go to the chunked big part
     unsigned chunk;    // edges of a big entry per warp grab
+    bool finish;       // sssp_finish_kernel ends the search (and writes the outputs)
+    double refuse;     // a parent edge this long is beyond the bucket ring
     // Renumbered search (both set) or not (both nullptr): the CSR is in the
     // search's numbering, roots and outputs in the caller's; perm maps a
     // caller's vertex to the search's, inv back.  Parents in pack are the
@@ -1038,7 +1062,7 @@ __global__ void __launch_bounds__(SSSP_THREADS, SSSP_MIN_BLOCKS) sssp_persistent
     SsspCtl *c = a.ctl;
     __shared__ float s_bnd[RING + 1];
     __shared__ float s_sub[SUB + 1];
-    __shared__ bool s_tiny_ok;
+    __shared__ bool s_tiny_ok, s_stop;
     constexpr int WARPS = SSSP_THREADS / 32;
     __shared__ unsigned s_fbuf[WARPS][STAGE_F], s_sbuf[WARPS][STAGE_S], s_rbuf[WARPS][RING * STAGE_R];
     __shared__ unsigned s_fcnt[WARPS], s_scnt[WARPS], s_rcnt[WARPS][RING];
@@ -1121,8 +1145,12 @@ __global__ void __launch_bounds__(SSSP_THREADS, SSSP_MIN_BLOCKS) sssp_persistent
             bool ok = a.td != nullptr;
             for (int j = 0; j < SUB && ok; ++j) ok = __fadd_rn(s_sub[j], a.tiny) >= s_sub[j + 1];
             s_tiny_ok = ok;
+            s_stop = a.finish && e_total - settled_entries <= max(FINISH_ENTRIES, e_total >> FINISH_SHIFT);
         }
         __syncthreads();
+        // Little left (every block sees the same counts): sssp_finish_kernel
+        // goes on from the ring queues.
+        if (s_stop) break;
         PushCtx x;
         x.st = stage;
         x.bucket = bucket;
@@ -1389,11 +1417,290 @@ __global__ void __launch_bounds__(SSSP_THREADS, SSSP_MIN_BLOCKS) sssp_persistent
     // Every distance is final (the last heavy phase ended at a grid barrier).
     // Outputs not written as vertices settled are written here: every
     // vertex, or with pre-filled outputs the reached ones.
-    if (!sparse_out) {
+    if (!sparse_out && !a.finish) {
         for (uint64_t v = gtid; v < a.n; v += nthreads) {
             const unsigned long long p = __ldcg(&a.pack[v]);
             if (p != UNREACHED || !prefilled) write_out(a, (unsigned)v, p);
         }
+    }
+}
+
+// ---- the end of a search ----------------------------------------------------
+// Every vertex waiting in a ring queue relaxes its whole row; so does, in the
+// next round, every vertex whose distance dropped, until none does.  That is
+// the same fixed point as the buckets', hence the same distances, and the
+// same parents: every vertex relaxes its row after its last decrease.
+//
+// A round's list holds (vertex, first unit): the units (edges >> ush) of all
+// rows lie end to end, so the edges of a round, not its vertices, are what
+// the warps share out, in chunks of 32 edges and up.  A round is then one
+// chain of a few dependent round trips however few and however long its
+// rows are (about 10 us; the time is latency, not traffic).
+
+constexpr unsigned FIN_CHUNK = 256;  // most units a warp takes at once
+
+// A warp's staging slice of the next list: vertices and the units of their
+// rows.
+struct FinStage {
+    unsigned *v, *d, *cnt;
+};
+constexpr unsigned FIN_STAGE = 64;
+
+// Entries of a slice to slots [base >> 32, ...) of the list, each with its
+// first unit.  All 32 lanes call it.
+__device__ __forceinline__ bool fin_write(const FinStage &q, unsigned c, unsigned long long base, unsigned *Lv,
+                                          unsigned *Lb, uint64_t n) {
+    const bool ok = (base >> 32) + c <= n;
+    if (ok) {
+        unsigned u = (unsigned)base;
+        for (unsigned i0 = 0; i0 < c; i0 += 32) {
+            const unsigned i = i0 + lane_id();
+            const unsigned d = i < c ? q.d[i] : 0u;
+            const unsigned incl = warp_incl_scan(d);
+            if (i < c) {
+                Lv[(base >> 32) + i] = q.v[i];
+                Lb[(base >> 32) + i] = u + incl - d;
+            }
+            u += __shfl_sync(FULL, incl, 31);
+        }
+    }
+    __syncwarp();
+    return ok;
+}
+
+// entries << 32 | units of a slice.  All 32 lanes call it.
+__device__ __forceinline__ unsigned long long fin_staged(const FinStage &q) {
+    const unsigned c = *q.cnt;
+    unsigned t = 0;
+    for (unsigned i = lane_id(); i < c; i += 32) t += q.d[i];
+    return ((unsigned long long)c << 32) | warp_sum(t);
+}
+
+// Queues v for the next round (once: its frontier stamp) for every lane with
+// `want`.  A full slice goes to the list with one atomic, which hands out
+// slots and first units in the same order.  All 32 lanes call it.
+__device__ __forceinline__ void fin_push(const SsspArgs &a, const FinStage &q, bool want, unsigned v, unsigned pid,
+                                         unsigned ush, unsigned *Lv, unsigned *Lb, unsigned long long *ctr) {
+    uint64_t len = 0;
+    if (want) len = __ldg(&a.rowptr[v + 1]) - __ldg(&a.rowptr[v]);
+    want = want && atomicExch(&a.fstamp[v], pid) != pid && len;
+    const unsigned mask = __ballot_sync(FULL, want);
+    if (!mask) return;
+    unsigned c = *q.cnt;
+    if (c + __popc(mask) > FIN_STAGE) {
+        const unsigned long long pk = fin_staged(q);
+        unsigned long long base = 0;
+        if (lane_id() == 0) base = atomicAdd(ctr, pk);
+        if (!fin_write(q, c, __shfl_sync(FULL, base, 0), Lv, Lb, a.n))
+            atomicOr(&a.ctl->error, DEVERR_CAPACITY | site_bit(SITE_PUSH));
+        c = 0;
+    }
+    if (want) {
+        const unsigned i = c + __popc(mask & lanemask_lt());
+        q.v[i] = v;
+        q.d[i] = (unsigned)((len + (1u << ush) - 1) >> ush);
+    }
+    __syncwarp();
+    if (lane_id() == 0) *q.cnt = c + __popc(mask);
+    __syncwarp();
+}
+
+// The entry of a list that holds unit e: the last of its cnt entries whose
+// first unit is at most e.  32 probes at a time.  All 32 lanes call it.
+__device__ __forceinline__ unsigned fin_find(const unsigned *Lb, unsigned cnt, unsigned e) {
+    unsigned lo = 0, hi = cnt;
+    while (hi - lo > 1) {  // warp-uniform
+        const unsigned step = (hi - lo + 31) / 32;
+        const uint64_t i = lo + (uint64_t)step * lane_id();
+        const bool le = i < hi && __ldcg(&Lb[i]) <= e;
+        const unsigned m = __ballot_sync(FULL, le) | 1u;
+        lo += step * (31 - __clz(m));
+        hi = (unsigned)min((uint64_t)hi, (uint64_t)lo + step);
+    }
+    return lo;
+}
+
+__global__ void __launch_bounds__(SSSP_THREADS, 3) sssp_finish_kernel(SsspArgs a) {
+    constexpr int WARPS = SSSP_THREADS / 32;
+    SsspCtl *c = a.ctl;
+    __shared__ unsigned s_v[WARPS][FIN_STAGE], s_d[WARPS][FIN_STAGE], s_cnt[WARPS];
+    __shared__ unsigned s_pend[WARPS][64];
+    __shared__ unsigned long long s_pk[WARPS];
+    const unsigned lane = lane_id(), wid = threadIdx.x >> 5;
+    const uint64_t gtid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const uint64_t nthreads = (uint64_t)gridDim.x * blockDim.x;
+    if (lane == 0) s_cnt[wid] = 0;
+    __syncwarp();
+    const FinStage q{s_v[wid], s_d[wid], &s_cnt[wid]};
+    const unsigned pid0 = (unsigned)ld_volatile(&c->phases);
+    const unsigned long long e_total = __ldg(&a.rowptr[a.n]);
+    // Units of 2^ush edges keep a list's total in 32 bits (rows round up).
+    unsigned ush = 0;
+    while ((e_total >> ush) + (ush ? a.n : 0) > 0xffffffffull) ++ush;
+    const float inf = __int_as_float(0x7f800000);
+    unsigned epoch = 0, round = 0, n_edges = 0, n_low = 0;
+    if (ld_volatile(&c->error)) return;  // the buckets failed: nothing to go on from
+
+    for (;; ++round) {
+        const unsigned s_cur = round % 3, s_nxt = (round + 1) % 3, s_clr = (round + 2) % 3;
+        const unsigned pid = pid0 + round;
+        unsigned *Lv = (round & 1) ? a.F[0] : a.F[1], *Lb = (round & 1) ? a.FB[0] : a.FB[1];
+        unsigned long long *ctr = &c->fin[s_nxt];
+        const unsigned long long pk = round ? ld_volatile(&c->fin[s_cur]) : 0ull;
+        const unsigned cnt = (unsigned)(pk >> 32), units = (unsigned)pk;
+        if (round && !units) break;
+        if (cnt > a.n) {  // every block reads the same size
+            atomicOr(&c->error, DEVERR_CAPACITY | site_bit(SITE_LIST_F));
+            break;
+        }
+        if (gtid == 0) {
+            c->fin[s_clr] = 0;
+            c->fgrab[s_clr] = 0;
+        }
+        if (round == 0) {
+            // The vertices of the ring queues that are not settled.  A vertex
+            // may sit in several (one per bucket its distance fell to).
+            for (int r = 0; r < RING; ++r) {
+                const unsigned len = ld_volatile(&c->sn.ring_len[r]);
+                const unsigned *R = a.ring + (uint64_t)r * a.n;
+                for (uint64_t b = gtid - lane; b < len; b += nthreads) {
+                    const uint64_t i = b + lane;
+                    bool ok = false;
+                    unsigned v = 0;
+                    if (i < len) {
+                        v = __ldcg(&R[i]);
+                        ok = pack_dist(__ldcg(&a.pack[v])) < inf && !((__ldcg(&a.settled[v >> 5]) >> (v & 31)) & 1u);
+                    }
+                    fin_push(a, q, ok, v, pid, ush, Lv, Lb, ctr);
+                }
+            }
+        } else {
+            const unsigned *L = (round & 1) ? a.F[1] : a.F[0], *B = (round & 1) ? a.FB[1] : a.FB[0];
+            // Neighbouring chunks go to different SMs, so that a short list spreads.
+            const unsigned nw = gridDim.x * WARPS, wg = wid * gridDim.x + blockIdx.x;
+            const unsigned C = min(FIN_CHUNK, ((units - 1) / nw / 32 + 1) * 32), nch = (units - 1) / C + 1;
+            unsigned np = 0;  // this warp's lowered vertices waiting in s_pend (below 32 between steps)
+            for (unsigned ch = wg; ch < nch;) {
+                unsigned next = nch;  // asked for while this chunk is worked on
+                if (nch > nw && lane == 0) next = nw + atomicAdd(&c->fgrab[s_cur], 1u);
+                const unsigned u0 = ch * C, u1 = units - u0 > C ? u0 + C : units;
+                for (unsigned lo = fin_find(B, cnt, u0);; lo += 32) {
+                    const unsigned i = lo + lane;
+                    const bool in = i < cnt;
+                    const unsigned ub = in ? __ldcg(&B[i]) : units, u = in ? __ldcg(&L[i]) : 0u;
+                    uint64_t rb = 0;
+                    unsigned deg = 0;
+                    float du = 0.0f;
+                    if (ub < u1) {  // this chunk's part of the row
+                        const uint64_t re = __ldg(&a.rowptr[u + 1]);
+                        rb = __ldg(&a.rowptr[u]);
+                        du = pack_dist(__ldcg(&a.pack[u]));
+                        const uint64_t cs = ub < u0 ? (uint64_t)(u0 - ub) << ush : 0;
+                        const uint64_t ce = min(re - rb, (uint64_t)(u1 - ub) << ush);
+                        deg = ce > cs ? (unsigned)(ce - cs) : 0u;
+                        rb += cs;
+                    }
+                    const unsigned incl = warp_incl_scan(deg), total = __shfl_sync(FULL, incl, 31), excl = incl - deg;
+                    for (unsigned e0 = 0; e0 < total; e0 += 64) {
+                        unsigned ev[2], eu[2];
+                        float cand[2];
+                        unsigned long long cur[2];
+#pragma unroll
+                        for (int t = 0; t < 2; ++t) {
+                            const unsigned e = e0 + 32 * t + lane;
+                            const bool has = e < total;
+                            const int j = warp_owner(excl, has ? e : total - 1);
+                            eu[t] = __shfl_sync(FULL, u, j);
+                            const uint64_t at = __shfl_sync(FULL, rb, j) + (e - __shfl_sync(FULL, excl, j));
+                            const float d = __shfl_sync(FULL, du, j);
+                            ev[t] = has ? (unsigned)__ldg(&a.col[at]) : 0u;
+                            cand[t] = has ? __fadd_rn(d, __ldg(&a.w[at])) : inf;
+                            n_edges += has;
+                        }
+#pragma unroll
+                        for (int t = 0; t < 2; ++t) {
+                            if (ev[t] >= a.n) {  // not a vertex: report it, touch nothing
+                                atomicOr(&c->error, DEVERR_RANGE);
+                                ev[t] = 0;
+                                cand[t] = inf;
+                            }
+                            cur[t] = e0 + 32 * t + lane < total ? __ldcg(&a.pack[ev[t]]) : 0ull;
+                        }
+#pragma unroll
+                        for (int t = 0; t < 2; ++t) {
+                            const unsigned long long w = ((unsigned long long)__float_as_uint(cand[t]) << 32) | eu[t];
+                            bool low = false;
+                            if (w < cur[t]) {
+                                const unsigned long long old = atomicMin(&a.pack[ev[t]], w);
+                                low = w < old && (old >> 32) != (w >> 32);
+                                if (low && !(cand[t] < inf)) {
+                                    if (cand[t] == inf) atomicOr(&c->error, DEVERR_RING);
+                                    low = false;  // as in the buckets: no distance to go on from
+                                }
+                            }
+                            const unsigned m = __ballot_sync(FULL, low);
+                            if (low) s_pend[wid][np + __popc(m & lanemask_lt())] = ev[t];
+                            np += __popc(m);
+                            n_low += low;
+                            __syncwarp();
+                            if (np >= 32) {  // 32 pushes at once: their loads and atomics serve a full warp
+                                np -= 32;
+                                const unsigned v = s_pend[wid][np + lane];
+                                __syncwarp();
+                                fin_push(a, q, true, v, pid, ush, Lv, Lb, ctr);
+                            }
+                        }
+                    }
+                    if (cnt - lo <= 32 || __shfl_sync(FULL, ub, 31) >= u1) break;
+                }
+                ch = __shfl_sync(FULL, next, 0);
+            }
+            fin_push(a, q, lane < np, lane < np ? s_pend[wid][lane] : 0u, pid, ush, Lv, Lb, ctr);
+        }
+        // The slices' rest: one range of the list per block.
+        const unsigned long long mine = fin_staged(q);
+        if (lane == 0) s_pk[wid] = mine;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            unsigned long long t = 0;
+            for (int w = 0; w < WARPS; ++w) {
+                const unsigned long long m = s_pk[w];
+                s_pk[w] = t;
+                t += m;
+            }
+            const unsigned long long base = t ? atomicAdd(ctr, t) : 0ull;
+            for (int w = 0; w < WARPS; ++w) s_pk[w] += base;
+        }
+        __syncthreads();
+        if (!fin_write(q, (unsigned)(mine >> 32), s_pk[wid], Lv, Lb, a.n))
+            atomicOr(&c->error, DEVERR_CAPACITY | site_bit(SITE_FLUSH));
+        if (lane == 0) s_cnt[wid] = 0;
+        __syncwarp();
+        if (a.nblocks == 1) {
+            __syncthreads();
+            if (ld_volatile(&c->error)) return;
+        } else if (!grid_sync(&c->fbar, &c->error, epoch, a.nblocks, a.limit_ns)) {
+            return;
+        }
+        if (gtid == 0) trace_phase(c, pid, 7, cnt);
+    }
+    const unsigned long long te = warp_sum((unsigned long long)n_edges), tl = warp_sum((unsigned long long)n_low);
+    if (lane == 0 && te) atomicAdd(&c->n_edges, te);
+    if (lane == 0 && tl) atomicAdd(&c->n_improved, tl);
+    // Every distance is final: the outputs, and the edges on shortest paths
+    // that no ring of buckets reaches, which the buckets must refuse.
+    const bool prefilled = __ldcg((const unsigned long long *)&a.prefilled->dist) == (unsigned long long)a.dist &&
+                           __ldcg((const unsigned long long *)&a.prefilled->pred) == (unsigned long long)a.pred;
+    for (uint64_t v = gtid; v < a.n; v += nthreads) {
+        const unsigned long long p = __ldcg(&a.pack[v]);
+        if (p != UNREACHED || !prefilled) write_out(a, (unsigned)v, p);
+        if (p != UNREACHED && (double)pack_dist(p) >= a.refuse &&
+            (double)pack_dist(p) - (double)pack_dist(__ldcg(&a.pack[(unsigned)p])) >= a.refuse)
+            atomicOr(&c->error, DEVERR_RING);
+    }
+    if (gtid == 0) {
+        c->buckets += 1;
+        c->phases = pid0 + round;
     }
 }
 
@@ -1786,6 +2093,10 @@ static int sssp_launch(const uint64_t *d_rowstarts, const int32_t *d_col, const 
     a.nblocks = (unsigned)blocks;
     a.limit_ns = wait_limit_ns();
     a.check_opens = p.check_opens != 0;
+    // Asking for pulls or sub-buckets by their thresholds, or for checked
+    // opens, asks for buckets to the end.
+    a.finish = p.pull == 0.0f && p.sub_min == 0 && !p.check_opens;
+    a.refuse = (double)p.delta * RING * (1.0 + 1e-5);
     a.big_deg = p.big_deg ? (unsigned)p.big_deg : sssp_tile(nverts);
     a.chunk = p.chunk ? (unsigned)p.chunk : sssp_tile(nverts);
     a.perm = p.perm;
@@ -1794,6 +2105,7 @@ static int sssp_launch(const uint64_t *d_rowstarts, const int32_t *d_col, const 
         sssp_small_kernel<<<1, SSSP_THREADS, 0, st>>>(a);
     } else if (blocks == 1) {  // nothing to co-schedule: a plain launch
         sssp_persistent_kernel<<<1, SSSP_THREADS, 0, st>>>(a);
+        if (a.finish) sssp_finish_kernel<<<1, SSSP_THREADS, 0, st>>>(a);
     } else {
         // Cooperative launch.  (An L2 persisting window over the settled
         // bitmap and the packed distances, as the BFS has for its bitmaps,
@@ -1801,6 +2113,10 @@ static int sssp_launch(const uint64_t *d_rowstarts, const int32_t *d_col, const 
         void *args[] = {&a};
         G5_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)sssp_persistent_kernel, dim3(blocks),
                                                 dim3(SSSP_THREADS), args, 0, st));
+        // Three blocks an SM fit of either kernel, so the same grid does.
+        if (a.finish)
+            G5_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)sssp_finish_kernel, dim3(blocks), dim3(SSSP_THREADS),
+                                                    args, 0, st));
     }
     G5_CUDA_TRY(cudaGetLastError());
     return G5_OK;
