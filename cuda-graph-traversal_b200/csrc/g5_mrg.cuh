@@ -43,8 +43,13 @@ G5_HD uint32_t mrg_fold(uint64_t x) {
     return (uint32_t)(x >= MRG_P ? x - MRG_P : x);
 }
 
+// One step's sum stays below 2^58 (MRG_X < 2^27, MRG_Y < 2^17, words below
+// 2^31), so one fold leaves less than 2 p in 32 bits and the smaller of r and
+// r - p (mod 2^32) is the residue.
 G5_HD uint32_t mrg_next(MrgState &s) {
-    uint32_t n = mrg_fold((uint64_t)MRG_X * s.z[0] + (uint64_t)MRG_Y * s.z[4]);
+    const uint64_t x = (uint64_t)MRG_X * s.z[0] + (uint64_t)MRG_Y * s.z[4];
+    const uint32_t r = ((uint32_t)x & MRG_P) + (uint32_t)(x >> 31);
+    const uint32_t n = r < r - MRG_P ? r : r - MRG_P;
     s.z[4] = s.z[3];
     s.z[3] = s.z[2];
     s.z[2] = s.z[1];
@@ -68,15 +73,22 @@ G5_HD void mrg_apply(const MrgMatrix &M, MrgState &s) {
     }
 }
 
-// Quadrant of one Kronecker level with the reference's initiator
+// One Kronecker level with the reference's initiator
 // (src/graph_generation.cu:114-143, SPK_NOISE_LEVEL 0): draws below
 // (2^31-1) mod 10^4 are rejected, the rest reduced mod 10^4 and split at
-// 1900 (quadrant 1), 3800 (2), 9500 (0), else 3.
-G5_HD int kron_quadrant(MrgState &s) {
+// 1900 (quadrant 1), 3800 (2), 9500 (0), else 3; on the diagonal quadrant 2
+// is folded onto 1 (cuda_make_one_edge, :186-207).  Appends the level's bit
+// to each endpoint (most significant level first, so equal prefixes are the
+// diagonal).
+template <class U>
+G5_HD void kron_level(MrgState &s, U &src, U &dst) {
     uint32_t u = mrg_next(s);
     while (u < MRG_P % 10000u) u = mrg_next(s);
     u %= 10000u;
-    return u < 1900u ? 1 : u < 3800u ? 2 : u < 9500u ? 0 : 3;
+    const bool right = u < (src == dst ? 3800u : 1900u), both = u >= 9500u;  // quadrants 1 and 3
+    const bool down = !right && u < 3800u;                                   // quadrant 2
+    src = src + src + (U)(down || both);
+    dst = dst + dst + (U)(right || both);
 }
 
 G5_HD uint64_t bit_reverse64(uint64_t x) {
@@ -116,23 +128,29 @@ G5_HD float mrg_unit_float(uint32_t u) {
 }
 
 // One Graph500 edge from the stream that starts at s: one quadrant per
-// level, most significant bit first, folding the lower-left quadrant onto the
-// upper-right while on the diagonal (cuda_make_one_edge,
+// level, most significant bit first (cuda_make_one_edge,
 // src/graph_generation.cu:186-207), both endpoints scrambled, then the
-// weight drawn from the same stream (:225-238).
+// weight drawn from the same stream (:225-238).  Up to 32 levels the
+// endpoints are built in 32 bits.  The levels are the generator's time
+// (integer issue, about 42 slots a level; 5 levels unrolled keep the state's
+// words in place instead of moving four of them a step): 50 M edges at SCALE
+// 22 take 1.70 ms, with 64-bit endpoints and general reductions 2.85.
+template <class U>
+G5_HD void kron_levels(MrgState &s, int log_n, uint64_t &src_out, uint64_t &dst_out) {
+    U src = 0, dst = 0;
+#ifdef __CUDA_ARCH__
+#pragma unroll 5
+#endif
+    for (int lvl = 0; lvl < log_n; ++lvl) kron_level(s, src, dst);
+    src_out = src;
+    dst_out = dst;
+}
+
 G5_HD void kron_edge(MrgState s, int log_n, uint64_t val0, uint64_t val1, uint64_t &src_out, uint64_t &dst_out,
                      float &w_out) {
-    uint64_t src = 0, dst = 0;
-    for (int lvl = log_n - 1; lvl >= 0; --lvl) {
-        const int q = kron_quadrant(s);
-        uint64_t so = (uint64_t)(q >> 1), to = (uint64_t)(q & 1);
-        if (src == dst && so > to) {
-            so = 0;
-            to = 1;
-        }
-        src |= so << lvl;
-        dst |= to << lvl;
-    }
+    uint64_t src, dst;
+    if (log_n <= 32) kron_levels<uint32_t>(s, log_n, src, dst);
+    else kron_levels<uint64_t>(s, log_n, src, dst);
     src_out = kron_scramble(src, log_n, val0, val1);
     dst_out = kron_scramble(dst, log_n, val0, val1);
     w_out = mrg_unit_float(mrg_next(s));
