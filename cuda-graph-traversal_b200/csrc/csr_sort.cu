@@ -573,43 +573,14 @@ __global__ void row_lengths_kernel(const uint64_t *__restrict__ rowstarts, uint6
     }
 }
 
-// Sort keys of every entry: (~deg(neighbour), neighbour) in the (col, w)
-// slots the row sort orders by, so sorted rows list their neighbours by
-// decreasing degree, ties by index.
-__global__ void degree_keys_kernel(const int *__restrict__ col, uint64_t e, const unsigned *__restrict__ deg,
-                                   uint64_t n, int *__restrict__ ka, float *__restrict__ kb,
-                                   unsigned *__restrict__ err) {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < e; i += stride) {
-        const unsigned v = (unsigned)__ldg(&col[i]);
-        if (v >= n) atomicOr(err, SORTERR_RANGE);
-        ka[i] = (int)(0xffffffffu - (v < n ? __ldg(&deg[v]) : 0u));
-        kb[i] = __uint_as_float(v);
-    }
-}
-
 // --------------------------------------------------- SSSP vertex numbering
 
-// Sort keys of the vertex order: (~degree, index) in the (col, w) slots of
-// one row of n entries.
-__global__ void vertex_order_keys_kernel(const unsigned *__restrict__ deg, uint64_t n, int *__restrict__ ka,
-                                         float *__restrict__ kb) {
+// The new rows' lengths.
+__global__ void vertex_lengths_kernel(const unsigned *__restrict__ inv, const unsigned *__restrict__ deg, uint64_t n,
+                                      unsigned *__restrict__ len2) {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += stride) {
-        ka[v] = (int)(0xffffffffu - __ldg(&deg[v]));
-        kb[v] = __uint_as_float((unsigned)v);
-    }
-}
-
-// perm[inv[i]] = i, and the new rows' lengths.
-__global__ void vertex_perm_kernel(const unsigned *__restrict__ inv, const unsigned *__restrict__ deg, uint64_t n,
-                                   unsigned *__restrict__ perm, unsigned *__restrict__ len2) {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-        const unsigned o = __ldg(&inv[i]);
-        perm[o] = (unsigned)i;
-        len2[i] = __ldg(&deg[o]);
-    }
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
+        len2[i] = __ldg(&deg[__ldg(&inv[i])]);
 }
 
 // Row i of the renumbered copy = row inv[i] of the source, in the same
@@ -1359,6 +1330,392 @@ static int sort_grid(int per_sm) {
     return di.sms * per_sm;
 }
 
+// The radix passes' function attributes, once per device.
+static int radix_smem_setup() {
+    static bool smem_set[64] = {};
+    int dev = 0;
+    G5_CUDA_TRY(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64 || !smem_set[dev]) {
+        G5_CUDA_TRY(cudaFuncSetAttribute(csr_radix_pass_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)RX_SMEM));
+        G5_CUDA_TRY(cudaFuncSetAttribute(csr_radix_pass_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)RX_SMEM));
+        if (dev >= 0 && dev < 64) smem_set[dev] = true;
+    }
+    return G5_OK;
+}
+
+// ------------------------------------------------------------ vertex order
+
+// The vertices by decreasing degree, ties by index: a stable LSD radix sort
+// of (~degree, index) by the passes of the CSR build, skipping the digits in
+// which no two degrees differ (one row sort of all vertices, ten merge
+// passes, took 0.95 ms for 3 M vertices).
+struct OrderWork {
+    unsigned long long *hist, *base, *total;
+    unsigned *cnt;
+    unsigned long long *status;
+    unsigned long long *ka, *kb;
+    unsigned *va, *vb;
+};
+constexpr int ORDER_PASSES = 4;
+
+static OrderWork carve_order(Carver &c, uint64_t n) {
+    OrderWork w;
+    w.hist = c.take<unsigned long long>(ORDER_PASSES * RX_BINS);
+    w.base = c.take<unsigned long long>(ORDER_PASSES * RX_BINS);
+    w.total = c.take<unsigned long long>(2);
+    w.cnt = c.take<unsigned>(64);
+    w.status = c.take<unsigned long long>((n + RX_TILE - 1) / RX_TILE * RX_BINS);
+    w.ka = c.take<unsigned long long>(n);
+    w.kb = c.take<unsigned long long>(n);
+    w.va = c.take<unsigned>(n);
+    w.vb = c.take<unsigned>(n);
+    return w;
+}
+
+__global__ void __launch_bounds__(256) vertex_order_keys_kernel(const unsigned *__restrict__ deg, uint64_t n,
+                                                                unsigned long long *__restrict__ key,
+                                                                unsigned *__restrict__ val,
+                                                                unsigned long long *__restrict__ hist) {
+    __shared__ unsigned s_h[ORDER_PASSES * RX_BINS];
+    for (int i = threadIdx.x; i < ORDER_PASSES * RX_BINS; i += blockDim.x) s_h[i] = 0;
+    __syncthreads();
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t v = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += stride) {
+        const unsigned k = 0xffffffffu - __ldg(&deg[v]);
+        key[v] = k;
+        val[v] = (unsigned)v;
+#pragma unroll
+        for (int p = 0; p < ORDER_PASSES; ++p) atomicAdd(&s_h[p * RX_BINS + ((k >> (RX_BITS * p)) & (RX_BINS - 1))], 1u);
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < ORDER_PASSES * RX_BINS; i += blockDim.x)
+        if (s_h[i]) atomicAdd(&hist[i], (unsigned long long)s_h[i]);
+}
+
+__global__ void vertex_perm_kernel(const unsigned *__restrict__ order, uint64_t n, unsigned *__restrict__ inv,
+                                   unsigned *__restrict__ perm) {
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+        const unsigned o = __ldg(&order[i]);
+        inv[i] = o;
+        perm[o] = (unsigned)i;
+    }
+}
+
+// inv = the order, perm its inverse.  Synchronises (the digit counts).
+static int vertex_order(const unsigned *deg, uint64_t n, const OrderWork &w, unsigned *perm, unsigned *inv,
+                        cudaStream_t st) {
+    const int grid = sort_grid(8);
+    const uint64_t ntiles = (n + RX_TILE - 1) / RX_TILE;
+    G5_CUDA_TRY(cudaMemsetAsync(w.hist, 0, ORDER_PASSES * RX_BINS * sizeof(unsigned long long), st));
+    G5_CUDA_TRY(cudaMemsetAsync(w.cnt, 0, 64 * sizeof(unsigned), st));
+    G5_CUDA_TRY(cudaMemsetAsync(w.status, 0, ntiles * RX_BINS * sizeof(unsigned long long), st));
+    vertex_order_keys_kernel<<<grid, 256, 0, st>>>(deg, n, w.ka, w.va, w.hist);
+    csr_radix_scan_kernel<<<1, RX_BINS, 0, st>>>(w.hist, ORDER_PASSES, w.base, w.total);
+    unsigned long long hist[ORDER_PASSES * RX_BINS];
+    G5_CUDA_TRY(cudaMemcpyAsync(hist, w.hist, sizeof hist, cudaMemcpyDeviceToHost, st));
+    G5_CUDA_TRY(cudaStreamSynchronize(st));
+    int rc = radix_smem_setup();
+    if (rc) return rc;
+    RxPass a{};
+    a.n = n;
+    a.E = n;
+    a.status = w.status;
+    a.err = &w.cnt[RXC_ERR];
+    a.limit_ns = wait_limit_ns();
+    a.ntiles = ntiles;
+    a.kin = w.ka;
+    a.vin = w.va;
+    a.kout = w.kb;
+    a.vout = w.vb;
+    for (int p = 0; p < ORDER_PASSES; ++p) {
+        bool one = false;  // every key has the same digit: nothing to do
+        for (int d = 0; d < RX_BINS; ++d) one = one || hist[p * RX_BINS + d] == n;
+        if (one) continue;
+        a.shift = RX_BITS * p;
+        a.epoch = (unsigned long long)(p + 1);
+        a.base = w.base + p * RX_BINS;
+        a.hist = w.hist + p * RX_BINS;
+        a.tilectr = &w.cnt[RXC_TILES + p];
+        csr_radix_pass_kernel<false><<<(unsigned)ntiles, RX_THREADS, RX_SMEM, st>>>(a);
+        unsigned long long *k = (unsigned long long *)a.kin;
+        unsigned *v = (unsigned *)a.vin;
+        a.kin = a.kout;
+        a.vin = a.vout;
+        a.kout = k;
+        a.vout = v;
+    }
+    vertex_perm_kernel<<<grid, 256, 0, st>>>(a.vin, n, inv, perm);
+    G5_CUDA_TRY(cudaGetLastError());
+    return G5_OK;
+}
+
+// -------------------------------------------------- rows by vertex order
+//
+// g5_csr_degree_order: every row's neighbours by their place in the vertex
+// order.  Keys are the places, 32 bits and no payload (the neighbour is
+// inv[place]), so a block sorts up to 4096 of them by LSD radix in shared
+// memory, one pass per 8 bits of a place, where 64-bit bitonic sorts took 78
+// steps.  3 M vertices, 96 M entries: 3.3 ms for the rows and 0.15 for the
+// order, with 64-bit (~degree, neighbour) keys 6.7.
+//   up to 32 entries: a warp, bitonic in registers; up to 256: a warp, bitonic
+//   in shared memory; up to 4096: a block; longer rows: tiles of 4096 sorted
+//   by a block each, then merge passes over the whole grid.
+
+constexpr unsigned RK_TILE = 4096;
+constexpr int RK_PER = RK_TILE / SORT_THREADS;  // keys a thread holds
+static_assert(RK_TILE == BIG_TILE && RK_TILE == SORT_SMEM_KEYS, "one tile size for the row classes");
+
+__device__ __forceinline__ unsigned row_place(const int *__restrict__ col, const unsigned *__restrict__ perm,
+                                              uint64_t n, uint64_t i, unsigned *err) {
+    const unsigned v = (unsigned)__ldg(&col[i]);
+    if (v >= n) {
+        atomicOr(err, SORTERR_RANGE);
+        return 0;
+    }
+    return __ldg(&perm[v]);
+}
+
+// s[0 .. L) sorted by the whole block (L <= RK_TILE, keys below 2^bits).
+__device__ void block_radix(unsigned *s, unsigned (*wcnt)[RX_BINS], unsigned *wsum, unsigned L, int bits) {
+    constexpr int WARPS = SORT_THREADS / 32;
+    static_assert(SORT_THREADS == RX_BINS, "one thread per digit");
+    const unsigned tid = threadIdx.x, lane = lane_id(), wid = tid >> 5;
+    const unsigned per = (L + SORT_THREADS - 1) / SORT_THREADS;  // block-uniform, 1 .. RK_PER
+    const unsigned b0 = wid * per * 32 + lane;
+    unsigned *wc = wcnt[wid];
+    for (int shift = 0; shift < bits; shift += RX_BITS) {
+        for (int i = lane; i < RX_BINS; i += 32) wc[i] = 0;
+        __syncwarp();
+        unsigned key[RK_PER], rank[RK_PER / 2];
+#pragma unroll
+        for (int k = 0; k < RK_PER; ++k) {
+            key[k] = 0;
+            if (k < (int)per) {
+                const unsigned i = b0 + 32 * k;
+                const bool ok = i < L;
+                key[k] = ok ? s[i] : 0u;
+                const unsigned d = ok ? (key[k] >> shift) & (RX_BINS - 1) : RX_BINS;
+                const unsigned peers = __match_any_sync(FULL, d);
+                const unsigned leader = __ffs(peers) - 1;
+                unsigned c = 0;
+                if (ok && lane == leader) {
+                    c = wc[d];
+                    wc[d] = c + __popc(peers);
+                }
+                c = __shfl_sync(FULL, c, leader);
+                const unsigned r = c + __popc(peers & lanemask_lt());
+                rank[k / 2] = (k & 1) ? rank[k / 2] | r << 16 : r;
+                __syncwarp();
+            }
+        }
+        __syncthreads();
+        unsigned tot = 0;
+#pragma unroll
+        for (int q = 0; q < WARPS; ++q) {
+            const unsigned c = wcnt[q][tid];
+            wcnt[q][tid] = tot;
+            tot += c;
+        }
+        const unsigned incl = warp_incl_scan(tot);
+        if (lane == 31) wsum[wid] = incl;
+        __syncthreads();
+        unsigned off = incl - tot;
+#pragma unroll
+        for (int q = 0; q < WARPS; ++q)
+            if (q < (int)wid) off += wsum[q];
+#pragma unroll
+        for (int q = 0; q < WARPS; ++q) wcnt[q][tid] += off;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < RK_PER; ++k) {
+            if (k < (int)per && b0 + 32 * k < L)
+                s[wc[(key[k] >> shift) & (RX_BINS - 1)] + ((rank[k / 2] >> (16 * (k & 1))) & 0xffffu)] = key[k];
+        }
+        __syncthreads();
+    }
+}
+
+__global__ void __launch_bounds__(256) rank_rows_warp_kernel(const uint64_t *__restrict__ rowstarts, uint64_t n,
+                                                             const int *__restrict__ col,
+                                                             const unsigned *__restrict__ perm,
+                                                             const unsigned *__restrict__ inv, int *__restrict__ out,
+                                                             unsigned *__restrict__ mid, unsigned *__restrict__ big,
+                                                             unsigned *__restrict__ cnt) {
+    __shared__ unsigned s_rows[8][WARP_SMEM_KEYS];
+    unsigned *sk = s_rows[threadIdx.x >> 5];
+    unsigned *err = &cnt[2];
+    const unsigned lane = lane_id();
+    const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
+    for (uint64_t v0 = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; v0 < n; v0 += nw * 32) {
+        const uint64_t v = v0 + lane;
+        const uint64_t b = v < n ? rowstarts[v] : 0, len = v < n ? rowstarts[v + 1] - b : 0;
+        const bool is_mid = len > WARP_SMEM_KEYS && len <= RK_TILE, is_big = len > RK_TILE;
+        const unsigned pm = warp_append(&cnt[0], is_mid);
+        if (is_mid) mid[pm] = (unsigned)v;
+        const unsigned pb = warp_append(&cnt[1], is_big);
+        if (is_big) big[pb] = (unsigned)v;
+        if (len == 1) out[b] = (int)__ldg(&inv[row_place(col, perm, n, b, err)]);
+        unsigned todo = __ballot_sync(FULL, len >= 2 && len <= WARP_SMEM_KEYS);
+        while (todo) {
+            const int l = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const uint64_t rb = __shfl_sync(FULL, b, l);
+            const unsigned rl = (unsigned)__shfl_sync(FULL, len, l);
+            if (rl <= 32) {
+                unsigned k = lane < rl ? row_place(col, perm, n, rb + lane, err) : ~0u;
+#pragma unroll
+                for (int size = 2; size <= 32; size <<= 1) {
+#pragma unroll
+                    for (int j = size >> 1; j > 0; j >>= 1) {
+                        const unsigned o = __shfl_xor_sync(FULL, k, j);
+                        const bool up = (lane & size) == 0, lower = (lane & j) == 0;
+                        k = (lower == up) ? min(k, o) : max(k, o);
+                    }
+                }
+                if (lane < rl) out[rb + lane] = (int)__ldg(&inv[k]);
+                continue;
+            }
+            unsigned P = 64;
+            while (P < rl) P <<= 1;
+            for (unsigned i = lane; i < P; i += 32) sk[i] = i < rl ? row_place(col, perm, n, rb + i, err) : ~0u;
+            __syncwarp();
+            for (unsigned size = 2; size <= P; size <<= 1) {
+                for (unsigned j = size >> 1; j > 0; j >>= 1) {
+                    for (unsigned t = lane; t < P / 2; t += 32) {
+                        const unsigned i = 2 * t - (t & (j - 1)), q = i + j;
+                        const unsigned x = sk[i], y = sk[q];
+                        if ((x > y) == ((i & size) == 0)) {
+                            sk[i] = y;
+                            sk[q] = x;
+                        }
+                    }
+                    __syncwarp();
+                }
+            }
+            for (unsigned i = lane; i < rl; i += 32) out[rb + i] = (int)__ldg(&inv[sk[i]]);
+            __syncwarp();
+        }
+    }
+}
+
+__global__ void __launch_bounds__(SORT_THREADS) rank_rows_mid_kernel(const uint64_t *__restrict__ rowstarts,
+                                                                     const unsigned *__restrict__ mid,
+                                                                     unsigned *__restrict__ cnt, uint64_t n, int bits,
+                                                                     const int *__restrict__ col,
+                                                                     const unsigned *__restrict__ perm,
+                                                                     const unsigned *__restrict__ inv,
+                                                                     int *__restrict__ out) {
+    __shared__ unsigned s[RK_TILE], s_wcnt[SORT_THREADS / 32][RX_BINS], s_wsum[SORT_THREADS / 32];
+    const unsigned nrows = cnt[0];
+    for (unsigned k = blockIdx.x; k < nrows; k += gridDim.x) {
+        const unsigned v = mid[k];
+        const uint64_t rb = rowstarts[v];
+        const unsigned L = (unsigned)(rowstarts[v + 1] - rb);
+        for (unsigned i = threadIdx.x; i < L; i += blockDim.x) s[i] = row_place(col, perm, n, rb + i, &cnt[2]);
+        __syncthreads();
+        block_radix(s, s_wcnt, s_wsum, L, bits);
+        for (unsigned i = threadIdx.x; i < L; i += blockDim.x) out[rb + i] = (int)__ldg(&inv[s[i]]);
+        __syncthreads();
+    }
+}
+
+// Every tile of every big row sorted into key[].
+__global__ void __launch_bounds__(SORT_THREADS) rank_rows_chunks_kernel(const uint64_t *__restrict__ rowstarts,
+                                                                        const unsigned *__restrict__ big,
+                                                                        unsigned nbig, const uint64_t *__restrict__ tp,
+                                                                        uint64_t ntiles, uint64_t n, int bits,
+                                                                        const int *__restrict__ col,
+                                                                        const unsigned *__restrict__ perm,
+                                                                        unsigned *__restrict__ key,
+                                                                        unsigned *__restrict__ err) {
+    __shared__ unsigned s[RK_TILE], s_wcnt[SORT_THREADS / 32][RX_BINS], s_wsum[SORT_THREADS / 32];
+    for (uint64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        const unsigned k = tile_row(tp, nbig, t);
+        const uint64_t rb = rowstarts[big[k]], L = rowstarts[big[k] + 1] - rb;
+        const uint64_t c0 = (t - tp[k]) * RK_TILE;
+        const unsigned cl = L - c0 < RK_TILE ? (unsigned)(L - c0) : RK_TILE;
+        for (unsigned i = threadIdx.x; i < cl; i += blockDim.x) s[i] = row_place(col, perm, n, rb + c0 + i, err);
+        __syncthreads();
+        block_radix(s, s_wcnt, s_wsum, cl, bits);
+        for (unsigned i = threadIdx.x; i < cl; i += blockDim.x) key[rb + c0 + i] = s[i];
+        __syncthreads();
+    }
+}
+
+// One merge pass over the big rows longer than R (csr_merge_pass_kernel on
+// 32-bit keys); a row whose runs already cover it is passed over, so a row's
+// sorted keys are in `src` of the first pass after its last (rank_rows_finish).
+__global__ void __launch_bounds__(SORT_THREADS) rank_rows_merge_kernel(const uint64_t *__restrict__ rowstarts,
+                                                                       const unsigned *__restrict__ big,
+                                                                       unsigned nbig, const uint64_t *__restrict__ tp,
+                                                                       uint64_t ntiles, uint64_t R,
+                                                                       const unsigned *__restrict__ src,
+                                                                       unsigned *__restrict__ dst) {
+    __shared__ unsigned s[RK_TILE];
+    __shared__ uint64_t s_i[2];
+    for (uint64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        const unsigned k = tile_row(tp, nbig, t);
+        const uint64_t rb = rowstarts[big[k]], L = rowstarts[big[k] + 1] - rb;
+        if (L <= R) continue;  // the same t for the whole block
+        const uint64_t o = (t - tp[k]) * RK_TILE;
+        const uint64_t a0 = o / (2 * R) * (2 * R);
+        const uint64_t la = min(R, L - a0), b0 = a0 + la, lb = b0 < L ? min(R, L - b0) : 0;
+        const uint64_t d0 = o - a0, d1 = min(d0 + RK_TILE, la + lb);
+        if (threadIdx.x < 2) {
+            const uint64_t d = threadIdx.x ? d1 : d0;
+            s_i[threadIdx.x] = co_rank(
+                d, la, lb, [&](uint64_t i) { return src[rb + a0 + i]; }, [&](uint64_t j) { return src[rb + b0 + j]; });
+        }
+        __syncthreads();
+        const uint64_t i0 = s_i[0], i1 = s_i[1], j0 = d0 - i0, j1 = d1 - i1;
+        const unsigned na = (unsigned)(i1 - i0), nb = (unsigned)(j1 - j0);
+        for (unsigned q = threadIdx.x; q < na + nb; q += blockDim.x)
+            s[q] = q < na ? src[rb + a0 + i0 + q] : src[rb + b0 + j0 + (q - na)];
+        __syncthreads();
+        // Each thread merges RK_PER outputs in registers, back through shared
+        // memory, so that the stores are coalesced.
+        const unsigned q0 = threadIdx.x * RK_PER;
+        unsigned x[RK_PER];
+        if (q0 < na + nb) {
+            const unsigned *A = s, *B = s + na;
+            unsigned i = (unsigned)co_rank(
+                q0, na, nb, [&](uint64_t y) { return A[y]; }, [&](uint64_t y) { return B[y]; });
+            unsigned j = q0 - i;
+#pragma unroll
+            for (int q = 0; q < RK_PER; ++q) {
+                if (q0 + q < na + nb) {
+                    const bool takeA = j >= nb || (i < na && A[i] <= B[j]);
+                    x[q] = takeA ? A[i++] : B[j++];
+                }
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < RK_PER; ++q)
+            if (q0 + q < na + nb) s[q0 + q] = x[q];
+        __syncthreads();
+        for (unsigned q = threadIdx.x; q < na + nb; q += blockDim.x) dst[rb + a0 + d0 + q] = s[q];
+        __syncthreads();
+    }
+}
+
+// The big rows' sorted keys (in key0 after an even number of passes) as neighbours.
+__global__ void rank_rows_finish_kernel(const uint64_t *__restrict__ rowstarts, const unsigned *__restrict__ big,
+                                        unsigned nbig, const uint64_t *__restrict__ tp, uint64_t ntiles,
+                                        const unsigned *__restrict__ key0, const unsigned *__restrict__ key1,
+                                        const unsigned *__restrict__ inv, int *__restrict__ out) {
+    for (uint64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
+        const unsigned k = tile_row(tp, nbig, t);
+        const uint64_t rb = rowstarts[big[k]], L = rowstarts[big[k] + 1] - rb;
+        const unsigned *key = merge_passes(L) % 2 == 0 ? key0 : key1;
+        const uint64_t c0 = (t - tp[k]) * RK_TILE, c1 = min(c0 + RK_TILE, L);
+        for (uint64_t i = c0 + threadIdx.x; i < c1; i += blockDim.x) out[rb + i] = (int)__ldg(&inv[key[rb + i]]);
+    }
+}
+
 }  // namespace g5
 
 using namespace g5;
@@ -1550,16 +1907,8 @@ extern "C" int g5_csr_radix_fill(const uint64_t *d_edges, const float *d_weights
         G5_CUDA_TRY(cudaStreamSynchronize(st));
         return G5_OK;
     }
-    static bool smem_set[64][2] = {};  // the function attributes, once per device
-    int dev = 0;
-    G5_CUDA_TRY(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64 || !smem_set[dev][0]) {
-        G5_CUDA_TRY(cudaFuncSetAttribute(csr_radix_pass_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)RX_SMEM));
-        G5_CUDA_TRY(cudaFuncSetAttribute(csr_radix_pass_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)RX_SMEM));
-        if (dev >= 0 && dev < 64) smem_set[dev][0] = true;
-    }
+    int rc = radix_smem_setup();
+    if (rc) return rc;
     const uint64_t t_first = (nedges + RX_EDGE_TILE - 1) / RX_EDGE_TILE, t_rest = (E + RX_TILE - 1) / RX_TILE;
     G5_CUDA_TRY(cudaMemsetAsync(w.status, 0, t_first * RX_BINS * sizeof(unsigned long long), st));
     RxPass a{};
@@ -1617,8 +1966,7 @@ extern "C" int g5_csr_radix_fill(const uint64_t *d_edges, const float *d_weights
         sw.cnt = w.scnt;
         csr_sort_mid_kernel<<<sort_grid(4), SORT_THREADS, 0, st>>>(w.runs, w.rmid, w.scnt, d_col, d_w, d_col64);
         G5_CUDA_TRY(cudaGetLastError());
-        int rc = sort_big_rows(w.runs, d_col, d_w, d_col64, sw, 1, st);
-        if (rc) return rc;
+        if ((rc = sort_big_rows(w.runs, d_col, d_w, d_col64, sw, 1, st))) return rc;
         G5_CUDA_TRY(cudaStreamSynchronize(st));
     }
     return G5_OK;
@@ -1669,9 +2017,42 @@ extern "C" int g5_csr_dedupe_copy(const uint64_t *d_rowstarts, const int32_t *d_
     return G5_OK;
 }
 
+// Scratch of g5_csr_degree_order: the row lists and big-row tiles as in the
+// canonical sort, the vertex order's, degrees, perm and inv, and two arrays
+// of 32-bit keys for the big rows.
+struct RankWork {
+    SortWork w;  // mid, big, cnt, tcnt, tp, scan of these arrays
+    OrderWork order;
+    unsigned *deg, *perm, *inv, *key[2];
+    uint64_t bytes;
+};
+
+static RankWork carve_rank(void *base, uint64_t n, uint64_t e) {
+    Carver c(base);
+    RankWork r;
+    const uint64_t T = max_tiles(n, e);
+    r.w = SortWork{};
+    r.w.tmax = T;
+    r.w.mid = c.take<unsigned>(n);
+    r.w.big = c.take<unsigned>(n);
+    r.w.cnt = c.take<unsigned>(64);
+    r.w.tcnt = c.take<unsigned>(T);
+    r.w.tp = c.take<uint64_t>(n + 1);
+    r.w.scan = c.take<uint64_t>(scan_scratch_words(T > n ? T : n));
+    r.order = carve_order(c, n);
+    r.deg = c.take<unsigned>(n);
+    r.perm = c.take<unsigned>(n);
+    r.inv = c.take<unsigned>(n);
+    r.key[0] = c.take<unsigned>(e);
+    r.key[1] = c.take<unsigned>(e);
+    r.bytes = c.used;
+    return r;
+}
+
 extern "C" int g5_csr_degree_order_workspace_size(uint64_t nverts, uint64_t nentries, uint64_t *bytes) {
     G5_CHECK_ARG(bytes, "g5_csr_degree_order_workspace_size: bytes is NULL");
-    *bytes = carve_sort(nullptr, nverts, nentries).bytes + align_up(nentries * 4, 256) + align_up(nverts * 4, 256);
+    // never less than the canonical sort's: callers reuse one scratch for both
+    *bytes = std::max(carve_sort(nullptr, nverts, nentries).bytes, carve_rank(nullptr, nverts, nentries).bytes);
     return G5_OK;
 }
 
@@ -1687,45 +2068,70 @@ extern "C" int g5_csr_degree_order(const uint64_t *d_rowstarts, const int32_t *d
     g5_csr_degree_order_workspace_size(nverts, nentries, &need);
     if (work_bytes < need) return set_error(G5_ERR_WORKSPACE, "g5_csr_degree_order: workspace too small");
     if (nentries == 0) return G5_OK;
-    SortWork w = carve_sort(d_work, nverts, nentries);
-    int *ka = (int *)((char *)d_work + w.bytes);
-    unsigned *deg = (unsigned *)((char *)ka + align_up(nentries * 4, 256));
+    const RankWork r = carve_rank(d_work, nverts, nentries);
+    const SortWork &w = r.w;
+    const int bits = vertex_bits(nverts);
     cudaStream_t st = (cudaStream_t)stream;
-    G5_CUDA_TRY(cudaMemsetAsync(&w.cnt[2], 0, sizeof(unsigned), st));
-    row_lengths_kernel<<<sort_grid(8), 256, 0, st>>>(d_rowstarts, nverts, deg);
-    degree_keys_kernel<<<sort_grid(8), 256, 0, st>>>(d_col, nentries, deg, nverts, ka, (float *)d_out_col, &w.cnt[2]);
-    G5_CUDA_TRY(cudaGetLastError());
-    int rc = sort_rows(d_rowstarts, nverts, ka, (float *)d_out_col, nullptr, w, st);
+    G5_CUDA_TRY(cudaMemsetAsync(w.cnt, 0, 64 * sizeof(unsigned), st));
+    row_lengths_kernel<<<sort_grid(8), 256, 0, st>>>(d_rowstarts, nverts, r.deg);
+    int rc = vertex_order(r.deg, nverts, r.order, r.perm, r.inv, st);
     if (rc) return rc;
-    unsigned errs = 0;
+    const uint64_t warps = (nverts + 31) / 32;
+    const int wblocks = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)sort_grid(8), (warps + 7) / 8));
+    rank_rows_warp_kernel<<<wblocks, 256, 0, st>>>(d_rowstarts, nverts, d_col, r.perm, r.inv, d_out_col, w.mid, w.big,
+                                                   w.cnt);
+    rank_rows_mid_kernel<<<sort_grid(6), SORT_THREADS, 0, st>>>(d_rowstarts, w.mid, w.cnt, nverts, bits, d_col, r.perm,
+                                                                r.inv, d_out_col);
+    G5_CUDA_TRY(cudaGetLastError());
+    unsigned nbig = 0;
+    uint64_t ntiles = 0;
+    unsigned long long maxlen = 0;
+    if ((rc = big_rows_prepare(d_rowstarts, w, 1, st, &nbig, &ntiles, &maxlen))) return rc;
+    if (nbig) {
+        const int grid = (int)std::min<uint64_t>(ntiles, (uint64_t)sort_grid(6));
+        rank_rows_chunks_kernel<<<grid, SORT_THREADS, 0, st>>>(d_rowstarts, w.big, nbig, w.tp, ntiles, nverts, bits,
+                                                               d_col, r.perm, r.key[0], &w.cnt[2]);
+        int from = 0;
+        for (uint64_t R = RK_TILE; R < maxlen; R <<= 1, from ^= 1)
+            rank_rows_merge_kernel<<<grid, SORT_THREADS, 0, st>>>(d_rowstarts, w.big, nbig, w.tp, ntiles, R,
+                                                                  r.key[from], r.key[from ^ 1]);
+        rank_rows_finish_kernel<<<grid, 256, 0, st>>>(d_rowstarts, w.big, nbig, w.tp, ntiles, r.key[0], r.key[1], r.inv,
+                                                      d_out_col);
+        G5_CUDA_TRY(cudaGetLastError());
+    }
+    unsigned errs = 0, rxerr = 0;
     G5_CUDA_TRY(cudaMemcpyAsync(&errs, &w.cnt[2], sizeof errs, cudaMemcpyDeviceToHost, st));
+    G5_CUDA_TRY(cudaMemcpyAsync(&rxerr, &r.order.cnt[RXC_ERR], sizeof rxerr, cudaMemcpyDeviceToHost, st));
     G5_CUDA_TRY(cudaStreamSynchronize(st));
+    if (rxerr) return set_error(G5_ERR_TIMEOUT, "g5_csr_degree_order: the vertex order's radix sort gave up");
     if (errs) return set_error(G5_ERR_INVALID, "g5_csr_degree_order: a column entry is not a vertex");
     return G5_OK;
 }
 
-// Scratch of g5_csr_sssp_renumber: the row sort's for one row of n
-// entries, the degrees and new lengths, the sort keys, a scan's scratch.
-static uint64_t renumber_bytes(uint64_t n, uint64_t *off_deg, uint64_t *off_len, uint64_t *off_ka,
-                               uint64_t *off_rs, uint64_t *off_scan) {
-    uint64_t b = align_up(carve_sort(nullptr, 1, n).bytes, 256);
-    *off_deg = b;
-    b += align_up(n * 4, 256);
-    *off_len = b;
-    b += align_up(n * 4, 256);
-    *off_ka = b;
-    b += align_up(n * 4, 256);
-    *off_rs = b;
-    b += 256;
-    *off_scan = b;
-    b += align_up(scan_scratch_words(n) * 8, 256);
-    return b;
+// Scratch of g5_csr_sssp_renumber: the vertex order's, the degrees and new
+// lengths, error flags, a scan's scratch.
+struct RenumberWork {
+    OrderWork order;
+    unsigned *deg, *len2, *err;
+    uint64_t *scan;
+    uint64_t bytes;
+};
+
+static RenumberWork carve_renumber(void *base, uint64_t n) {
+    Carver c(base);
+    RenumberWork w;
+    w.order = carve_order(c, n);
+    w.deg = c.take<unsigned>(n);
+    w.len2 = c.take<unsigned>(n);
+    w.err = c.take<unsigned>(64);
+    w.scan = c.take<uint64_t>(scan_scratch_words(n));
+    w.bytes = c.used;
+    return w;
 }
 
 extern "C" int g5_csr_sssp_renumber_workspace_size(uint64_t nverts, uint64_t *bytes) {
     G5_CHECK_ARG(bytes, "g5_csr_sssp_renumber_workspace_size: bytes is NULL");
-    uint64_t a, b, c, d, e;
-    *bytes = renumber_bytes(nverts, &a, &b, &c, &d, &e);
+    *bytes = carve_renumber(nullptr, nverts).bytes;
     return G5_OK;
 }
 
@@ -1739,38 +2145,27 @@ extern "C" int g5_csr_sssp_renumber(const uint64_t *d_rowstarts, const int32_t *
     G5_CHECK_ARG(d_rowstarts && d_light_deg && d_tiny_deg && d_perm && d_inv && d_rowstarts_out && d_light_out &&
                      d_tiny_out && d_work && (nentries == 0 || (d_col && d_w && d_col_out && d_w_out)),
                  "g5_csr_sssp_renumber: NULL argument");
-    uint64_t off_deg, off_len, off_ka, off_rs, off_scan;
-    if (work_bytes < renumber_bytes(nverts, &off_deg, &off_len, &off_ka, &off_rs, &off_scan))
-        return set_error(G5_ERR_WORKSPACE, "g5_csr_sssp_renumber: workspace too small");
-    char *base = (char *)d_work;
-    SortWork w = carve_sort(d_work, 1, nverts);
-    unsigned *deg = (unsigned *)(base + off_deg), *len2 = (unsigned *)(base + off_len);
-    int *ka = (int *)(base + off_ka);
-    uint64_t *rs1 = (uint64_t *)(base + off_rs), *scan = (uint64_t *)(base + off_scan);
+    const RenumberWork w = carve_renumber(d_work, nverts);
+    if (work_bytes < w.bytes) return set_error(G5_ERR_WORKSPACE, "g5_csr_sssp_renumber: workspace too small");
     cudaStream_t st = (cudaStream_t)stream;
     const int grid = sort_grid(8);
-    // The vertex order: decreasing degree, ties by index (a row sort of one
-    // row of n keys); inv = the order, perm its inverse.
-    const uint64_t one_row[2] = {0, nverts};
-    G5_CUDA_TRY(cudaMemcpyAsync(rs1, one_row, sizeof one_row, cudaMemcpyHostToDevice, st));
-    G5_CUDA_TRY(cudaMemsetAsync(&w.cnt[2], 0, sizeof(unsigned), st));
-    row_lengths_kernel<<<grid, 256, 0, st>>>(d_rowstarts, nverts, deg);
-    vertex_order_keys_kernel<<<grid, 256, 0, st>>>(deg, nverts, ka, (float *)d_inv);
-    G5_CUDA_TRY(cudaGetLastError());
-    int rc = sort_rows(rs1, 1, ka, (float *)d_inv, nullptr, w, st);
+    G5_CUDA_TRY(cudaMemsetAsync(w.err, 0, sizeof(unsigned), st));
+    row_lengths_kernel<<<grid, 256, 0, st>>>(d_rowstarts, nverts, w.deg);
+    int rc = vertex_order(w.deg, nverts, w.order, d_perm, d_inv, st);
     if (rc) return rc;
-    vertex_perm_kernel<<<grid, 256, 0, st>>>(d_inv, deg, nverts, d_perm, len2);
+    vertex_lengths_kernel<<<grid, 256, 0, st>>>(d_inv, w.deg, nverts, w.len2);
     G5_CUDA_TRY(cudaGetLastError());
-    if ((rc = scan_u32_to_u64(len2, nverts, d_rowstarts_out, scan, st))) return rc;
+    if ((rc = scan_u32_to_u64(w.len2, nverts, d_rowstarts_out, w.scan, st))) return rc;
     renumber_rows_kernel<<<grid, 256, 0, st>>>(d_rowstarts, d_col, d_w, d_light_deg, d_tiny_deg, nverts, d_perm, d_inv,
-                                               d_rowstarts_out, d_col_out, d_w_out, d_light_out, d_tiny_out,
-                                               &w.cnt[2]);
+                                               d_rowstarts_out, d_col_out, d_w_out, d_light_out, d_tiny_out, w.err);
     renumber_long_rows_kernel<<<grid, 256, 0, st>>>(d_rowstarts, d_col, d_w, nverts, d_perm, d_inv, d_rowstarts_out,
-                                                    d_col_out, d_w_out, &w.cnt[2]);
+                                                    d_col_out, d_w_out, w.err);
     G5_CUDA_TRY(cudaGetLastError());
-    unsigned errs = 0;
-    G5_CUDA_TRY(cudaMemcpyAsync(&errs, &w.cnt[2], sizeof errs, cudaMemcpyDeviceToHost, st));
+    unsigned errs = 0, rxerr = 0;
+    G5_CUDA_TRY(cudaMemcpyAsync(&errs, w.err, sizeof errs, cudaMemcpyDeviceToHost, st));
+    G5_CUDA_TRY(cudaMemcpyAsync(&rxerr, &w.order.cnt[RXC_ERR], sizeof rxerr, cudaMemcpyDeviceToHost, st));
     G5_CUDA_TRY(cudaStreamSynchronize(st));
+    if (rxerr) return set_error(G5_ERR_TIMEOUT, "g5_csr_sssp_renumber: the vertex order's radix sort gave up");
     if (errs) return set_error(G5_ERR_INVALID, "g5_csr_sssp_renumber: a column entry is not a vertex");
     return G5_OK;
 }
