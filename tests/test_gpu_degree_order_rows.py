@@ -30,11 +30,18 @@ def test_rows_of_every_class(cgt, n):
     src = np.repeat(np.arange(n), length)
     want = col[np.lexsort((place[col], src))]
     assert np.array_equal(g.bcol.cpu().numpy(), want)
-    # the renumbered copy uses the same order
-    g.tiny_deg = torch.zeros(n, dtype=torch.int32, device="cuda")
+    # the renumbered copy uses the same order; its rows are the rows, renamed
+    w = rng.random(e, dtype=np.float32)
+    light, tiny = rng.integers(0, 9, n).astype(np.int32), rng.integers(0, 9, n).astype(np.int32)
+    g.w, g.light_deg, g.tiny_deg = (torch.tensor(x, device="cuda") for x in (w, light, tiny))
     cgt.oned_graph_sssp_renumber(g)
-    assert np.array_equal(g.sr.perm.cpu().numpy(), place)
-    assert np.array_equal(place[g.sr.inv.cpu().numpy()], np.arange(n))
+    inv = g.sr.inv.cpu().numpy()
+    assert np.array_equal(g.sr.perm.cpu().numpy(), place) and np.array_equal(place[inv], np.arange(n))
+    at = np.argsort(place[src], kind="stable")
+    assert np.array_equal(g.sr.rowstarts.cpu().numpy(), np.concatenate([[0], np.cumsum(length[inv])]))
+    assert np.array_equal(g.sr.col.cpu().numpy(), place[col[at]]) and np.array_equal(g.sr.w.cpu().numpy(), w[at])
+    assert np.array_equal(g.sr.light_deg.cpu().numpy(), light[inv])
+    assert np.array_equal(g.sr.tiny_deg.cpu().numpy(), tiny[inv])
 
 
 def test_bad_column_is_reported(cgt):
