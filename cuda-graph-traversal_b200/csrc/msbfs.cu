@@ -60,8 +60,9 @@ constexpr unsigned long long MS_PREPARED = 0x51afd7ed558ccd1dull;
 
 struct MsCtl {
     g5_msbfs_stats res;
-    unsigned bar;
-    unsigned nheavy;   // H: positions [0, H) have more than MS_LIGHT entries
+    // The polled word and each level's cursors have lines of their own.
+    alignas(128) unsigned bar;
+    alignas(128) unsigned nheavy;   // H: positions [0, H) have more than MS_LIGHT entries
     unsigned nlight;   // L: positions [H, H + L) have 1..MS_LIGHT entries
     unsigned nchunks;  // chunks of the heavy rows
     unsigned long long prepared;  // MS_PREPARED once g5_msbfs_prepare ran
@@ -69,9 +70,9 @@ struct MsCtl {
     unsigned long long clean;     // MS_CLEAN when fr[0], fr[1] and both bitmaps are zero
     unsigned long long roots[MS_MAX_ROOTS];
     // per level slot (level % 3)
-    unsigned wgrab[3];
-    unsigned cgrab[3];
-    unsigned n_f[3];
+    alignas(128) unsigned wgrab[3];
+    alignas(128) unsigned cgrab[3];
+    alignas(128) unsigned n_f[3];
     unsigned long long m_f[3];
     unsigned live[3][MS_W];  // roots with a non-empty frontier at that level
     // trace
@@ -646,10 +647,19 @@ __device__ void ms_pull(const MsArgs &a, int s, const unsigned *F, unsigned *X, 
     // Light rows [H, H + L), one lane per vertex: 32 consecutive positions
     // have rows of about equal length.
     const unsigned H = ld_volatile(&c->nheavy), nl = ld_volatile(&c->nlight);
+    // Up to 128 per grab when every warp gets several: one cursor serves the
+    // whole grid (131 K grabs of 32 a level on 4.2 M vertices, 3 % of its time).
+    const unsigned grab = min(128u, max(32u, nl / (4 * gridDim.x * (blockDim.x >> 5)) & ~31u));
+    unsigned i0 = 0, left = 0;
     for (;;) {
-        unsigned i0 = 0;
-        if (lane == 0) i0 = atomicAdd(&c->wgrab[s], 32u);
-        i0 = __shfl_sync(FULL, i0, 0);
+        if (left == 0) {
+            if (lane == 0) i0 = atomicAdd(&c->wgrab[s], grab);
+            i0 = __shfl_sync(FULL, i0, 0);
+            left = grab;
+        } else {
+            i0 += 32;
+        }
+        left -= 32;
         if (i0 >= nl) break;
         if (i0 + lane >= nl) continue;
         const unsigned v = H + i0 + lane;
@@ -868,7 +878,7 @@ __device__ __forceinline__ uint64_t byte_mask_of_bits(unsigned s8) {
 constexpr int EX_V = 128;
 static_assert(EX_V == 4 * 32, "a warp's 32 threads take the 128 vertices four each");
 
-__global__ void __launch_bounds__(256, 2) ms_export_u8_kernel(const unsigned *__restrict__ seen,
+__global__ void __launch_bounds__(256, 4) ms_export_u8_kernel(const unsigned *__restrict__ seen,
                                                            const unsigned *__restrict__ planes,
                                                            const unsigned *__restrict__ pos, uint64_t n, int bits,
                                                            unsigned nroots, uint8_t *__restrict__ out) {
@@ -960,6 +970,16 @@ __global__ void __launch_bounds__(256, 2) ms_export_u8_kernel(const unsigned *__
         }
         __syncthreads();
     }
+}
+
+// Blocks of a batch by default: one an SM (a quarter of what fits) up to 2^19
+// vertices, two up to 2^20, then all that fit; where levels are short, more
+// blocks only crowd the cursors and the barrier.  256 roots: 16 K vertices 0.98
+// ms on 148 blocks, 1.11 on 296 and 1.15 on 592; 260 K 1.11, 1.17 and 1.43; 40
+// roots on 1 M 1.43, 1.45 and 1.65; 256 on 4.2 M 5.67, 3.60 and 3.28.
+static int ms_blocks(uint64_t nverts, int max_blocks) {
+    const int sm = std::max(1, max_blocks / 4);
+    return nverts <= (1ull << 19) ? sm : nverts <= (1ull << 20) ? 2 * sm : max_blocks;
 }
 
 static int ms_max_blocks(int *out) {
@@ -1054,7 +1074,7 @@ extern "C" int g5_msbfs_run(uint64_t nverts, uint64_t nentries, int depth_bits, 
                  "g5_msbfs_run: bad params");
     int max_blocks = 0;
     if ((rc = ms_max_blocks(&max_blocks))) return rc;
-    const int blocks = p.blocks > 0 ? std::min(p.blocks, max_blocks) : max_blocks;
+    const int blocks = p.blocks > 0 ? std::min(p.blocks, max_blocks) : ms_blocks(nverts, max_blocks);
     cudaStream_t st = (cudaStream_t)stream;
     DeviceInfo di;
     if ((rc = device_info(&di))) return rc;
@@ -1112,7 +1132,7 @@ extern "C" int g5_msbfs_depths_u8(const void *d_work, uint64_t work_bytes, uint6
     G5_CHECK_ARG(d_out && nroots >= 1 && nroots <= MS_MAX_ROOTS, "g5_msbfs_depths_u8: bad argument");
     DeviceInfo di;
     if ((rc = device_info(&di))) return rc;
-    ms_export_u8_kernel<<<di.sms * 2, 256, 0, (cudaStream_t)stream>>>(w.seen, w.planes, w.pos, nverts, depth_bits,
+    ms_export_u8_kernel<<<di.sms * 4, 256, 0, (cudaStream_t)stream>>>(w.seen, w.planes, w.pos, nverts, depth_bits,
                                                                        nroots, d_out);
     G5_CUDA_TRY(cudaGetLastError());
     return G5_OK;
@@ -1171,8 +1191,8 @@ extern "C" int g5_msbfs_grid(uint64_t nverts, int32_t *blocks, int32_t *max_bloc
     int rc = ms_max_blocks(&mb);
     if (rc) return rc;
     *max_blocks = mb;
-    // g5_msbfs_run launches every co-resident block by default; this is the
-    // grid a caller sharing the device should pass in params.blocks.
+    // For a caller sharing the device to pass in params.blocks (by default
+    // g5_msbfs_run takes the grid that is fastest alone, ms_blocks).
     *blocks = (int)std::min<uint64_t>(mb, std::max<uint64_t>(1, nverts / 1024));
     return G5_OK;
 }
