@@ -99,14 +99,16 @@ constexpr unsigned long long SPLIT_MIN = 1ull << 22, SPLIT_MIN_MULTI = 1ull << 2
 // of all.  What is left after the bucket that holds the hubs hangs off settled
 // vertices and is seldom lowered twice, but it went through some 20 buckets
 // of at least three phases, about 10 us each however small: with the finish
-// 600 K vertices take 1.1 ms instead of 1.5, 90 packed graphs 8.9 instead of
-// 11.7.  A search handed over at once relaxes each entry about five times,
-// which beats the buckets' phases up to about 2^20 entries (16 K vertices:
-// 0.24 ms, in buckets 0.67).  A kernel of its own because the bucketed one is
-// as large as it should get: with this loop inside, it spilled three times as
-// much.
-constexpr unsigned long long FINISH_ENTRIES = 1ull << 20;
-constexpr int FINISH_SHIFT = 2;
+// 600 K vertices take 1.0 ms instead of 1.5, 90 packed graphs 7.8 instead of
+// 11.7 (8.7 when a quarter of the entries is the line instead of half).  A
+// search handed over at once relaxes each entry about five times, which beats
+// the buckets' phases up to about 2^22 entries (16 K vertices 0.25 ms, in
+// buckets 0.67; 100 K vertices, 2^21.6 entries, 0.40 ms, in buckets first
+// 0.56; 200 K, 2^22.6, 0.75 and 0.69).  A kernel of its own because the
+// bucketed one is as large as it should get: with this loop inside, it
+// spilled three times as much.
+constexpr unsigned long long FINISH_ENTRIES = 1ull << 22;
+constexpr int FINISH_SHIFT = 1;
 constexpr float SSSP_PULL_RATIO = 1.0f;  // default heavy-phase pull threshold
 constexpr double PULL_WALK = 0.25;       // cost of a pull's bitmap walk, in CSR entries per vertex
 constexpr unsigned long long UNREACHED = ~0ull;

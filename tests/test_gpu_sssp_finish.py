@@ -38,13 +38,13 @@ def _ties(rng):
 
 
 def _kron(rng):
-    """2^17 vertices, 2^21 edges: buckets first, then the finish."""
-    u = v = np.zeros(1 << 21, np.int64)
+    """2^17 vertices, 2^22 edges: buckets first, then the finish."""
+    u = v = np.zeros(1 << 22, np.int64)
     for _ in range(17):
-        r = rng.random(1 << 21)
+        r = rng.random(1 << 22)
         u = u * 2 + (r >= 0.76)
         v = v * 2 + (((r >= 0.57) & (r < 0.76)) | (r >= 0.95))
-    return 1 << 17, np.stack([u, v], 1), 1.0 - rng.random(1 << 21, dtype=np.float32)
+    return 1 << 17, np.stack([u, v], 1), 1.0 - rng.random(1 << 22, dtype=np.float32)
 
 
 @pytest.mark.parametrize("make", [_fans, _path, _heavy, _ties, _kron])
