@@ -47,10 +47,13 @@ constexpr int BFS_THREADS = 256;
 // Defaults: edges of a long row taken by one warp, and the longest row a warp
 // expands by itself.  A warp step of 32 edges is a chain of a few dependent
 // round trips, so the two bound a short level: on 700 K vertices (a level of
-// 36 rows with 64 K edges) 128 / 256 takes 95 us, 256 / 256 103 and 256 /
-// 1024 139; on 34 M vertices 732, 742 and 758.
-constexpr unsigned BFS_CHUNK = 128;
-constexpr unsigned BFS_BIG_DEG = 256;
+// 36 rows with 64 K edges) 128 / 256 takes 95 us, 256 / 256 103 and 256 / 1024
+// 139.  In a wide top-down level the chunks' one cursor is the bound instead:
+// 37 M edges on 34 M vertices take 1.04 ms with 128 / 256 and 0.69 with 256 /
+// 1024, the defaults from BFS_TILE_VERTICES on.
+constexpr unsigned BFS_CHUNK = 128, BFS_CHUNK_LARGE = 256;
+constexpr unsigned BFS_BIG_DEG = 256, BFS_BIG_DEG_LARGE = 1024;
+constexpr uint64_t BFS_TILE_VERTICES = 1ull << 22;
 constexpr unsigned BFS_STAGE = 512;  // per-warp staging of the next queue (16 KiB shared per block)
 constexpr unsigned long long SOLO_EDGES = 4096;  // levels at most this wide run in block 0 alone
 constexpr int BFS_TRACE = 64;                    // levels recorded in the control block
@@ -1256,8 +1259,9 @@ static int bfs_launch(const BfsWork &w, const uint64_t *d_rowstarts, const int32
     a.xout = xout;  // only the one-block search exports by itself
     a.xcap = xcap;
     a.xcount_map = xcount_map;
-    a.big_deg = p.big_deg ? (unsigned)p.big_deg : BFS_BIG_DEG;
-    a.chunk = p.chunk ? (unsigned)p.chunk : BFS_CHUNK;
+    const bool large = nverts > BFS_TILE_VERTICES;
+    a.big_deg = p.big_deg ? (unsigned)p.big_deg : large ? BFS_BIG_DEG_LARGE : BFS_BIG_DEG;
+    a.chunk = p.chunk ? (unsigned)p.chunk : large ? BFS_CHUNK_LARGE : BFS_CHUNK;
     a.lane_entries = p.lane_entries ? (unsigned)p.lane_entries : BU_LANE_ENTRIES;
     a.top = p.top;
     static std::atomic<unsigned long long> next_seq{1};

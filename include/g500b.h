@@ -224,9 +224,10 @@ typedef struct g5_bfs_params {
                        3 = one lean block, top-down (a root in a small component; g5_bfs_query picks
                        it from the main-component bitmap)                                             */
     int32_t blocks; /* persistent grid size; 0 = by the graph's size, up to the whole device              */
-    /* Work tiles (0 = default; none changes a result, only the speed):                                  */
-    int32_t big_deg;      /* queue entries with more edges are cut into chunks across the grid (256)      */
-    int32_t chunk;        /* edges per chunk, a multiple of 32 up to 65536 (128)                          */
+    /* Work tiles (0 = default; none changes a result, only the speed).  Defaults in brackets: up to 2^22
+       vertices, beyond:                                                                                 */
+    int32_t big_deg;      /* queue entries with more edges are cut into chunks across the grid (256, 1024)*/
+    int32_t chunk;        /* edges per chunk, a multiple of 32 up to 65536 (128, 256)                     */
     int32_t lane_entries; /* bottom-up: entries of a row one lane scans before its warp joins, a multiple
                              of 4 up to 1024 (8)                                                          */
     /* Optional (NULL = none): top[v] = col[rowstarts[v]], the first entry of v's row in the column the
