@@ -76,7 +76,7 @@ struct BfsCtl {
     // for 4 K vertices instead of 71, and 134 for 700 K instead of 124).
     alignas(128) unsigned bar;  // grid barrier arrivals
     alignas(128) unsigned n_small[3];  // per level slot: queue entries of degree <= BIG_DEG
-    unsigned long long big[3];  //           big entries << 40 | their chunks
+    unsigned long long big[3];  //           big entries and their chunks (big_pack)
     unsigned grab[3];     //                 work cursor over the small part
     unsigned cgrab[3];    //                 work cursor over the big part's chunks
     unsigned found[3];    //                 vertices found by a bottom-up level
@@ -612,7 +612,7 @@ __global__ void __launch_bounds__(BFS_THREADS, 4) bfs_persistent_kernel(BfsArgs 
                 if (root_deg > a.big_deg) {
                     a.q[0][a.n - 1] = root;
                     a.base[0][0] = 0;
-                    c->big[0] = (1ull << BIG_SHIFT) | ((root_deg + a.chunk - 1) / a.chunk);
+                    c->big[0] = big_pack(1, (unsigned)((root_deg + a.chunk - 1) / a.chunk));
                 } else {
                     a.q[0][0] = root;
                     c->n_small[0] = 1;

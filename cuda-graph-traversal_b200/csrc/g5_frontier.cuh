@@ -10,7 +10,7 @@
 // chunks and every warp of the grid takes chunks from one counter, so no
 // vertex's edges serialise on one warp.  Big entries are
 // appended with one 64-bit atomicAdd per warp on a packed counter
-// (entry count << 40 | chunk count), which hands out slots and first-chunk
+// (entries and chunks, 32 bits each), which hands out slots and first-chunk
 // ids in the same order, so chunk bases are sorted by slot and a chunk id
 // maps back to its vertex by binary search.
 #pragma once
@@ -28,13 +28,21 @@ __host__ __device__ __forceinline__ unsigned grab_size(unsigned ns, unsigned lon
     unsigned long long g = ns / (4 * nwarps);
     return g < 1 ? 1u : g > cap ? cap : (unsigned)g;
 }
-constexpr int BIG_SHIFT = 40;
-constexpr unsigned long long BIG_LOW = (1ull << BIG_SHIFT) - 1;
+
+// The packed counter of a big part.  Neither half overflows: a list holds a
+// vertex at most once, so entries stay at or below n < 2^32 (a field of 24
+// bits wrapped on 2^25 vertices of degree 64 in chunks of 32: slot 0 handed
+// out twice, chunk bases out of order); and chunks stay below E / chunk + n,
+// which for chunks of 32 entries and up reaches 2^32 only where n or the
+// column (256 GB at E = 2^36) is larger than the device holds.
+constexpr int BIG_SHIFT = 32;
+__host__ __device__ constexpr unsigned long long big_pack(unsigned entries, unsigned chunks) {
+    return ((unsigned long long)entries << BIG_SHIFT) | chunks;
+}
+__host__ __device__ constexpr unsigned big_count(unsigned long long packed) { return (unsigned)(packed >> BIG_SHIFT); }
+__host__ __device__ constexpr unsigned big_chunks(unsigned long long packed) { return (unsigned)packed; }
 
 #ifdef __CUDACC__
-
-__device__ __forceinline__ unsigned big_count(unsigned long long packed) { return (unsigned)(packed >> BIG_SHIFT); }
-__device__ __forceinline__ unsigned long long big_chunks(unsigned long long packed) { return packed & BIG_LOW; }
 
 // Appends v, whose edge range to expand has `deg` entries, to list L of
 // capacity n (base[] = chunk bases of the big part): the small part when
@@ -59,13 +67,13 @@ __device__ __forceinline__ bool frontier_append(unsigned *L, unsigned *base, uin
         const unsigned total = __shfl_sync(FULL, incl, 31);
         const unsigned leader = __ffs(bmask) - 1;
         unsigned long long old = 0;
-        if (lane_id() == leader) old = atomicAdd(big, ((unsigned long long)__popc(bmask) << BIG_SHIFT) | total);
+        if (lane_id() == leader) old = atomicAdd(big, big_pack(__popc(bmask), total));
         old = __shfl_sync(FULL, old, leader);
         if (bg) {
-            const uint64_t j = (old >> BIG_SHIFT) + __popc(bmask & lanemask_lt());
+            const uint64_t j = (uint64_t)big_count(old) + __popc(bmask & lanemask_lt());
             if (j < n) {
                 L[n - 1 - j] = v;
-                base[j] = (unsigned)((old & BIG_LOW) + incl - nch);
+                base[j] = big_chunks(old) + incl - nch;
             } else {
                 ok = false;
             }

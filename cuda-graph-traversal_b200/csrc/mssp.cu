@@ -26,6 +26,7 @@
 // in the bucket) + 8 per active source (its word of the target, read, then
 // lowered when improved); per round 12 per queued vertex.
 #include "g5_common.cuh"
+#include "g5_frontier.cuh"
 
 namespace g5 {
 
@@ -45,7 +46,7 @@ struct MssCtl {
     unsigned bar;                    // grid barrier arrivals
     unsigned err;                    // DEVERR_* flags
     alignas(128) unsigned qlen[3];   // per round slot: vertices queued for the next round
-    unsigned long long big[3];       // per round slot: long-row items << 40 | their chunks
+    unsigned long long big[3];       // per round slot: long-row items and their chunks (big_pack)
     unsigned minb[3];                // per round slot: smallest pending bucket seen (a lower bound)
     unsigned long long sources[MSS_SOURCES];  // in the CSR's numbering
     g5_sssp_multi_stats res;
@@ -235,7 +236,6 @@ __global__ void __launch_bounds__(MSS_THREADS) mss_persistent_kernel(MssArgs a) 
     const uint64_t gtid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const uint64_t nthreads = (uint64_t)gridDim.x * blockDim.x;
     const uint64_t gwarp = gtid >> 5, nwarps = nthreads >> 5;
-    const unsigned long long cmask40 = (1ull << 40) - 1;
     unsigned long long entries = 0, scanned = 0;
     const unsigned lane = lane_id();
     unsigned nf = ld_volatile(&c->qlen[0]);
@@ -278,12 +278,12 @@ __global__ void __launch_bounds__(MSS_THREADS) mss_persistent_kernel(MssArgs a) 
                 a.ws.smask[i] = m;
                 const uint64_t deg = __ldg(&a.rowptr[u + 1]) - __ldg(&a.rowptr[u]);
                 if (deg > MSS_CHUNK && m) {
-                    const unsigned long long nch = (deg + MSS_CHUNK - 1) / MSS_CHUNK;
-                    const unsigned long long old = atomicAdd(&c->big[sl], (1ull << 40) | nch);
-                    const unsigned long long k = old >> 40;
+                    const unsigned nch = (unsigned)((deg + MSS_CHUNK - 1) / MSS_CHUNK);
+                    const unsigned long long old = atomicAdd(&c->big[sl], big_pack(1, nch));
+                    const unsigned k = big_count(old);
                     if (k < a.n) {
                         a.ws.items[k] = (unsigned)i;
-                        a.ws.ibase[k] = old & cmask40;
+                        a.ws.ibase[k] = big_chunks(old);
                     } else {
                         atomicOr(&c->err, DEVERR_CAPACITY);
                     }
@@ -306,8 +306,8 @@ __global__ void __launch_bounds__(MSS_THREADS) mss_persistent_kernel(MssArgs a) 
             if (m) mss_relax(a, u, m, b, e, bk, true, nxt, &c->qlen[sn], wmin, scanned);
         }
         const unsigned long long bg = ld_volatile(&c->big[sl]);
-        const unsigned nitems = (unsigned)min(bg >> 40, (unsigned long long)a.n);
-        const unsigned long long nchunks = nitems ? (bg & cmask40) : 0;
+        const unsigned nitems = (unsigned)min((uint64_t)big_count(bg), a.n);
+        const unsigned long long nchunks = nitems ? big_chunks(bg) : 0;
         for (unsigned long long ch = gwarp; ch < nchunks; ch += nwarps) {
             const unsigned k = mss_item_of(a.ws.ibase, nitems, ch);
             const unsigned i = __ldcg(&a.ws.items[k]);
