@@ -1413,9 +1413,11 @@ __global__ void vertex_perm_kernel(const unsigned *__restrict__ order, uint64_t 
     }
 }
 
-// inv = the order, perm its inverse.  Synchronises (the digit counts).
+// inv = the order, perm its inverse.  Synchronises twice: for the digit
+// counts and for the passes' error word, since a pass whose look-back gave up
+// leaves places of the order unwritten, and all that follows indexes by it.
 static int vertex_order(const unsigned *deg, uint64_t n, const OrderWork &w, unsigned *perm, unsigned *inv,
-                        cudaStream_t st) {
+                        cudaStream_t st, const char *who) {
     const int grid = sort_grid(8);
     const uint64_t ntiles = (n + RX_TILE - 1) / RX_TILE;
     G5_CUDA_TRY(cudaMemsetAsync(w.hist, 0, ORDER_PASSES * RX_BINS * sizeof(unsigned long long), st));
@@ -1456,6 +1458,12 @@ static int vertex_order(const unsigned *deg, uint64_t n, const OrderWork &w, uns
         a.kout = k;
         a.vout = v;
     }
+    G5_CUDA_TRY(cudaGetLastError());
+    unsigned err = 0;
+    G5_CUDA_TRY(cudaMemcpyAsync(&err, a.err, sizeof err, cudaMemcpyDeviceToHost, st));
+    G5_CUDA_TRY(cudaStreamSynchronize(st));
+    if (err & SORTERR_WAIT) return set_error(G5_ERR_TIMEOUT, "%s: a look-back wait of the vertex order gave up", who);
+    if (err) return set_error(G5_ERR_DEVICE, "%s: the vertex order is incomplete (flags 0x%x)", who, err);
     vertex_perm_kernel<<<grid, 256, 0, st>>>(a.vin, n, inv, perm);
     G5_CUDA_TRY(cudaGetLastError());
     return G5_OK;
@@ -2083,7 +2091,7 @@ extern "C" int g5_csr_degree_order(const uint64_t *d_rowstarts, const int32_t *d
     cudaStream_t st = (cudaStream_t)stream;
     G5_CUDA_TRY(cudaMemsetAsync(w.cnt, 0, 64 * sizeof(unsigned), st));
     row_lengths_kernel<<<sort_grid(8), 256, 0, st>>>(d_rowstarts, nverts, r.deg);
-    int rc = vertex_order(r.deg, nverts, r.order, r.perm, r.inv, st);
+    int rc = vertex_order(r.deg, nverts, r.order, r.perm, r.inv, st, "g5_csr_degree_order");
     if (rc) return rc;
     const uint64_t warps = (nverts + 31) / 32;
     const int wblocks = (int)std::max<uint64_t>(1, std::min<uint64_t>((uint64_t)sort_grid(8), (warps + 7) / 8));
@@ -2108,11 +2116,9 @@ extern "C" int g5_csr_degree_order(const uint64_t *d_rowstarts, const int32_t *d
                                                       d_out_col);
         G5_CUDA_TRY(cudaGetLastError());
     }
-    unsigned errs = 0, rxerr = 0;
+    unsigned errs = 0;
     G5_CUDA_TRY(cudaMemcpyAsync(&errs, &w.cnt[2], sizeof errs, cudaMemcpyDeviceToHost, st));
-    G5_CUDA_TRY(cudaMemcpyAsync(&rxerr, &r.order.cnt[RXC_ERR], sizeof rxerr, cudaMemcpyDeviceToHost, st));
     G5_CUDA_TRY(cudaStreamSynchronize(st));
-    if (rxerr) return set_error(G5_ERR_TIMEOUT, "g5_csr_degree_order: the vertex order's radix sort gave up");
     if (errs) return set_error(G5_ERR_INVALID, "g5_csr_degree_order: a column entry is not a vertex");
     return G5_OK;
 }
@@ -2160,7 +2166,7 @@ extern "C" int g5_csr_sssp_renumber(const uint64_t *d_rowstarts, const int32_t *
     const int grid = sort_grid(8);
     G5_CUDA_TRY(cudaMemsetAsync(w.err, 0, sizeof(unsigned), st));
     row_lengths_kernel<<<grid, 256, 0, st>>>(d_rowstarts, nverts, w.deg);
-    int rc = vertex_order(w.deg, nverts, w.order, d_perm, d_inv, st);
+    int rc = vertex_order(w.deg, nverts, w.order, d_perm, d_inv, st, "g5_csr_sssp_renumber");
     if (rc) return rc;
     renumber_vertices_kernel<<<grid, 256, 0, st>>>(d_inv, w.deg, d_light_deg, d_tiny_deg, nverts, w.len2, d_light_out,
                                                    d_tiny_out);
@@ -2169,11 +2175,9 @@ extern "C" int g5_csr_sssp_renumber(const uint64_t *d_rowstarts, const int32_t *
     renumber_entries_kernel<<<grid, 256, 0, st>>>(d_rowstarts, d_col, d_w, nverts, d_perm, d_inv, d_rowstarts_out,
                                                   d_col_out, d_w_out, w.err);
     G5_CUDA_TRY(cudaGetLastError());
-    unsigned errs = 0, rxerr = 0;
+    unsigned errs = 0;
     G5_CUDA_TRY(cudaMemcpyAsync(&errs, w.err, sizeof errs, cudaMemcpyDeviceToHost, st));
-    G5_CUDA_TRY(cudaMemcpyAsync(&rxerr, &w.order.cnt[RXC_ERR], sizeof rxerr, cudaMemcpyDeviceToHost, st));
     G5_CUDA_TRY(cudaStreamSynchronize(st));
-    if (rxerr) return set_error(G5_ERR_TIMEOUT, "g5_csr_sssp_renumber: the vertex order's radix sort gave up");
     if (errs) return set_error(G5_ERR_INVALID, "g5_csr_sssp_renumber: a column entry is not a vertex");
     return G5_OK;
 }
