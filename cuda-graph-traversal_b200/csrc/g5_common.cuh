@@ -157,6 +157,18 @@ __device__ __forceinline__ bool grid_sync(unsigned *count, unsigned *error, unsi
     return s_ok;
 }
 
+// A block barrier, then whether *error is set: one thread reads it and all
+// get its answer, since another block (or a faster warp) may set it between
+// two threads' reads, and threads that left alone would be missing from the
+// warp and block collectives of the others.
+__device__ __forceinline__ bool block_error(const unsigned *error) {
+    __shared__ unsigned s_err;
+    __syncthreads();
+    if (threadIdx.x == 0) s_err = ld_volatile(error);
+    __syncthreads();
+    return s_err != 0;
+}
+
 template <class T>
 __device__ __forceinline__ T warp_incl_scan(T x) {
 #pragma unroll

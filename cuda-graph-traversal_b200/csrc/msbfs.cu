@@ -765,7 +765,7 @@ __global__ void __launch_bounds__(MS_THREADS, 4) ms_persistent_kernel(MsArgs a) 
     unsigned epoch = 0;
     __shared__ unsigned s_live[MS_W];
     if (blockIdx.x == 0 && threadIdx.x == 0) c->t0 = globaltimer_ns();
-    if (ld_volatile(&c->res.error_flags)) return;  // the seed found a bad root or an unprepared workspace
+    if (block_error(&c->res.error_flags)) return;  // the seed found a bad root or an unprepared workspace
     int levels = 0, pull_levels = 0;
     unsigned long long fedges = 0;
     for (int level = 0;; ++level) {

@@ -833,8 +833,7 @@ __device__ __forceinline__ bool sssp_sync(const SsspArgs &a, unsigned &epoch, Ss
     if (a.nblocks == 1) {
         // One block (a search in a small component): the block barrier
         // orders every global write of the phase before the next phase.
-        __syncthreads();
-        if (ld_volatile(&a.ctl->error)) return false;
+        if (block_error(&a.ctl->error)) return false;
     } else if (!grid_sync(&a.ctl->bar, &a.ctl->error, epoch, a.nblocks, a.limit_ns)) {
         return false;
     }
@@ -1541,7 +1540,7 @@ __global__ void __launch_bounds__(SSSP_THREADS, 3) sssp_finish_kernel(SsspArgs a
     while ((e_total >> ush) + (ush ? a.n : 0) > 0xffffffffull) ++ush;
     const float inf = __int_as_float(0x7f800000);
     unsigned epoch = 0, round = 0, n_edges = 0, n_low = 0;
-    if (ld_volatile(&c->error)) return;  // the buckets failed: nothing to go on from
+    if (block_error(&c->error)) return;  // the buckets failed: nothing to go on from
 
     for (;; ++round) {
         const unsigned s_cur = round % 3, s_nxt = (round + 1) % 3, s_clr = (round + 2) % 3;
@@ -1679,8 +1678,7 @@ __global__ void __launch_bounds__(SSSP_THREADS, 3) sssp_finish_kernel(SsspArgs a
         if (lane == 0) s_cnt[wid] = 0;
         __syncwarp();
         if (a.nblocks == 1) {
-            __syncthreads();
-            if (ld_volatile(&c->error)) return;
+            if (block_error(&c->error)) return;
         } else if (!grid_sync(&c->fbar, &c->error, epoch, a.nblocks, a.limit_ns)) {
             return;
         }
