@@ -1620,12 +1620,9 @@ __global__ void __launch_bounds__(SSSP_THREADS, 3) sssp_finish_kernel(SsspArgs a
                         }
 #pragma unroll
                         for (int t = 0; t < 2; ++t) {
-                            if (ev[t] >= a.n) {  // not a vertex: report it, touch nothing
-                                atomicOr(&c->error, DEVERR_RANGE);
-                                ev[t] = 0;
-                                cand[t] = inf;
-                            }
-                            cur[t] = e0 + 32 * t + lane < total ? __ldcg(&a.pack[ev[t]]) : 0ull;
+                            const bool has = e0 + 32 * t + lane < total;
+                            if (ev[t] >= a.n) atomicOr(&c->error, DEVERR_RANGE);  // not a vertex: report it, touch nothing
+                            cur[t] = has && ev[t] < a.n ? __ldcg(&a.pack[ev[t]]) : 0ull;
                         }
 #pragma unroll
                         for (int t = 0; t < 2; ++t) {
