@@ -1889,6 +1889,7 @@ static SsspWork carve_sssp(void *base, uint64_t n) {
     return w;
 }
 
+// The largest grid of which both kernels of a search fit on the device.
 static int sssp_max_blocks(int *out) {
     static int cached[64] = {};
     DeviceInfo di;
@@ -1896,10 +1897,12 @@ static int sssp_max_blocks(int *out) {
     if (rc) return rc;
     if (!cached[di.device]) {
         if ((rc = persistent_kernel_setup((const void *)sssp_persistent_kernel))) return rc;
-        int per_sm = 0;
+        if ((rc = persistent_kernel_setup((const void *)sssp_finish_kernel))) return rc;
+        int buckets = 0, finish = 0;
         G5_CUDA_TRY(
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sssp_persistent_kernel, SSSP_THREADS, 0));
-        cached[di.device] = std::max(1, per_sm) * di.sms;
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&buckets, sssp_persistent_kernel, SSSP_THREADS, 0));
+        G5_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&finish, sssp_finish_kernel, SSSP_THREADS, 0));
+        cached[di.device] = std::max(1, std::min(buckets, finish)) * di.sms;
     }
     *out = cached[di.device];
     return G5_OK;
@@ -2110,8 +2113,7 @@ static int sssp_launch(const uint64_t *d_rowstarts, const int32_t *d_col, const 
         void *args[] = {&a};
         G5_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)sssp_persistent_kernel, dim3(blocks),
                                                 dim3(SSSP_THREADS), args, 0, st));
-        // Three blocks an SM fit of either kernel, so the same grid does.
-        if (a.finish)
+        if (a.finish)  // the same grid (sssp_max_blocks)
             G5_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)sssp_finish_kernel, dim3(blocks), dim3(SSSP_THREADS),
                                                     args, 0, st));
     }
