@@ -84,16 +84,19 @@ constexpr unsigned SSSP_GRAB = 32;
 // distance drops several times inside the sub-bucket then re-reads its light
 // row (weights only decide) but repeats none of its random relaxations.
 constexpr int SUB = 32;
-// The line: 8.4 M vertices, whose frontier reaches 25 M light entries, take
-// 6.2 ms split from 2^18 to 2^22 on and 7.1 unsplit; 2.1 M vertices, which
-// reach 6 M, 3.0 ms split at 2^20 to 2^22, 3.2 unsplit and 4.6 at 2^18, where
-// the sub-buckets' phases cost more than the repeated relaxations; 600 K,
-// which reach 1.5 M, 2.0 ms unsplit and 2.8 split at 2^20.
+// The line: sub-buckets cost some 20 windows of three phases and save repeated
+// relaxations, so they pay on graphs of many entries, and there from the
+// first phases on, before most repeats are made.  Split at 2^22 against not
+// split: 8.4 M vertices and 268 M entries 5.9 and 6.6 ms, 6 M and 192 M 4.0 and
+// 4.6, 3 M and 192 M 3.8 and 4.2; 5 M and 160 M 4.5 and 4.3, 4.2 M and 134 M 4.2 and
+// 3.6, 2 M and 64 M 3.4 and 1.9, 1 M and 64 M 2.3 and 1.7.  Below SPLIT_ENTRIES
+// only a frontier of SPLIT_MIN_FEW splits.
 // With many sources (packed graphs) a large frontier is many small ones, whose
 // vertices are seldom lowered again: 90 graphs with 167 M entries in all take
 // 13 ms unsplit and 18 split, so there the line is where it hardly matters.
 // Defaults; g5_sssp_params.sub_min overrides.
-constexpr unsigned long long SPLIT_MIN = 1ull << 22, SPLIT_MIN_MULTI = 1ull << 25;
+constexpr unsigned long long SPLIT_ENTRIES = 5ull << 25;
+constexpr unsigned long long SPLIT_MIN = 1ull << 22, SPLIT_MIN_FEW = 1ull << 25;
 // The bucketed kernel hands over to sssp_finish_kernel once the rows of the
 // vertices not settled hold at most FINISH_ENTRIES entries or 2^-FINISH_SHIFT
 // of all.  What is left after the bucket that holds the hubs hangs off settled
@@ -223,6 +226,7 @@ struct SsspArgs {
     float light;       // light edges: w < light (light >= delta)
     float pull_ratio;  // heavy phase pulls when its rows' entries >= pull_ratio x unsettled rows' entries; <= 0 never
     unsigned long long split_min;  // frontier light entries that start sub-buckets (~0: never)
+    unsigned long long split_entries;  // graphs of fewer entries start them at SPLIT_MIN_FEW
     unsigned long long *pack;
     unsigned *fstamp, *sstamp;
     // Queue stamps: the lowest bucket (rstamp) and sub-bucket (jstamp,
@@ -1307,7 +1311,7 @@ __global__ void __launch_bounds__(SSSP_THREADS, SSSP_MIN_BLOCKS) sssp_persistent
                 ++phase;
                 continue;
             }
-            if (!x.sub_mode && sp->f_entries[s_cur] >= a.split_min) {
+            if (!x.sub_mode && sp->f_entries[s_cur] >= (e_total < a.split_entries ? SPLIT_MIN_FEW : a.split_min)) {
                 // Split: the frontier goes to the sub-bucket queues of its
                 // distances; the bucket continues by sub-buckets in order.
                 x.sub_mode = true;
@@ -2068,7 +2072,8 @@ static int sssp_launch(const uint64_t *d_rowstarts, const int32_t *d_col, const 
     a.nroots = nroots;
     a.delta = p.delta;
     a.pull_ratio = p.pull == 0.0f ? SSSP_PULL_RATIO : p.pull;
-    a.split_min = p.sub_min == 0 ? (d_roots ? SPLIT_MIN_MULTI : SPLIT_MIN) : p.sub_min < 0 ? ~0ull : (unsigned long long)p.sub_min;
+    a.split_min = p.sub_min == 0 ? (d_roots ? SPLIT_MIN_FEW : SPLIT_MIN) : p.sub_min < 0 ? ~0ull : (unsigned long long)p.sub_min;
+    a.split_entries = p.sub_min == 0 ? SPLIT_ENTRIES : 0;
     a.pack = w.pack;
     a.fstamp = w.fstamp;
     a.sstamp = w.sstamp;

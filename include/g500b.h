@@ -416,8 +416,9 @@ typedef struct g5_sssp_params {
                        rows; 0 = default (1.0), < 0 = always push           */
     int32_t sub_min; /* once a bucket's light frontier holds this many light
                        CSR entries, the rest of the bucket runs in 32
-                       sub-buckets in distance order; 0 = default (2^22;
-                       2^25 with several sources), < 0 = never                                           */
+                       sub-buckets in distance order; 0 = default (2^22 on
+                       graphs of 5 x 2^25 CSR entries and more, 2^25 on
+                       smaller ones and with several sources), < 0 = never  */
     int32_t small;   /* 1: the source's component is small (outside the main
                        component): one lean block, label-correcting rounds,
                        same distances and parents; 0 = the bucketed search  */
