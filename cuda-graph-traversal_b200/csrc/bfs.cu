@@ -931,18 +931,21 @@ static BfsWork carve_bfs(void *base, uint64_t n) {
     return w;
 }
 
-// Largest co-resident grid of the persistent kernel on this device.
 // Blocks of a search by default: one per 256 vertices until each SM has one
-// (a quarter of what fits), from 2^20 vertices on one per 8192.  More blocks
-// than a level has work for only poll the barrier: 4 K vertices take 49 us on
-// 16 blocks, 50 on 148 and 71 on 592; 700 K 95, 97 and 124 on 148, 222 and
-// 592; 2.1 M 226, 175, 173 and 180 on 148, 296, 444 and 592; 34 M 775 on 444
-// and 719 on 592.
+// (a quarter of what fits), one per 4096 until it has two, and one per 8192 beyond.
+// More blocks than a level has work for only poll the barrier: 4 K vertices
+// take 49 us on 16 blocks, 50 on 148 and 71 on 592; 700 K 95, 97 and 124 on 148, 222
+// and 592; 34 M 775 on 444 and 719 on 592.  From 700 K on dense graphs need
+// more than one an SM: edge factor 64, 1 M vertices 335, 261, 230 and 232 us on
+// 148, 222, 296 and 592 (with 8 104, 103, 107 and 131); edge factor 16, 1.2 M
+// 225 on 148 and 179 on 293, 2 M 222, 179, 186 and 199 on 148, 296, 444 and 592.
 static int bfs_blocks(uint64_t nverts, int max_blocks) {
-    const uint64_t small = std::min<uint64_t>(nverts / 256, (uint64_t)std::max(1, max_blocks / 4));
+    const uint64_t sm = std::max(1, max_blocks / 4);
+    const uint64_t small = std::max(std::min(nverts / 256, sm), std::min(nverts / 4096, 2 * sm));
     return (int)std::min<uint64_t>(max_blocks, std::max<uint64_t>(1, std::max(small, nverts / 8192)));
 }
 
+// Largest co-resident grid of the persistent kernel on this device.
 static int bfs_max_blocks(int *out) {
     static int cached[64] = {};
     DeviceInfo di;
