@@ -972,14 +972,19 @@ __global__ void __launch_bounds__(256, 4) ms_export_u8_kernel(const unsigned *__
     }
 }
 
-// Blocks of a batch by default: one an SM (a quarter of what fits) up to 2^19
-// vertices, two up to 2^20, then all that fit; where levels are short, more
-// blocks only crowd the cursors and the barrier.  256 roots: 16 K vertices 0.98
-// ms on 148 blocks, 1.11 on 296 and 1.15 on 592; 260 K 1.11, 1.17 and 1.43; 40
-// roots on 1 M 1.43, 1.45 and 1.65; 256 on 4.2 M 5.67, 3.60 and 3.28.
-static int ms_blocks(uint64_t nverts, int max_blocks) {
+// Blocks of a batch by default: one an SM (a quarter of what fits) up to 2^25
+// CSR entries, two up to 2^26, three up to 3 x 2^25, then all that fit; where
+// levels are short, more blocks only crowd the cursors and the barrier.  256
+// roots on 148, 296, 444 and 592 blocks: 260 K vertices and 8 M entries 1.14, 1.34, 1.43
+// and 1.53 ms, 600 K and 19 M 1.64, 1.76, 1.86 and 2.06, 400 K and 51 M 1.69, 1.45, 1.54 and
+// 1.65, 600 K and 77 M 2.39, 2.04, 1.90 and 2.02, 1 M and 128 M 3.25, 2.39, 2.35 and 2.28.
+// (By vertices, as the BFS's grid, dense graphs got too few.)
+static int ms_blocks(uint64_t nentries, int max_blocks) {
     const int sm = std::max(1, max_blocks / 4);
-    return nverts <= (1ull << 19) ? sm : nverts <= (1ull << 20) ? 2 * sm : max_blocks;
+    return nentries <= (1ull << 25) ? sm
+         : nentries <= (1ull << 26) ? 2 * sm
+         : nentries <= (3ull << 25) ? 3 * sm
+                                    : max_blocks;
 }
 
 static int ms_max_blocks(int *out) {
@@ -1074,7 +1079,7 @@ extern "C" int g5_msbfs_run(uint64_t nverts, uint64_t nentries, int depth_bits, 
                  "g5_msbfs_run: bad params");
     int max_blocks = 0;
     if ((rc = ms_max_blocks(&max_blocks))) return rc;
-    const int blocks = p.blocks > 0 ? std::min(p.blocks, max_blocks) : ms_blocks(nverts, max_blocks);
+    const int blocks = p.blocks > 0 ? std::min(p.blocks, max_blocks) : ms_blocks(nentries, max_blocks);
     cudaStream_t st = (cudaStream_t)stream;
     DeviceInfo di;
     if ((rc = device_info(&di))) return rc;

@@ -68,6 +68,9 @@ cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3 g, dim3 b, void **args, size
 cudaError_t cudaLaunchCooperativeKernel(const void *fun, dim3 g, dim3 b, void **args, size_t s, cudaStream_t st) {
     return cudaLaunchKernel(fun, g, b, args, s, st);
 }
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *fun, void **args) {
+    return cudaLaunchKernel(fun, c->gridDim, c->blockDim, args, c->dynamicSmemBytes, c->stream);
+}
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int *n, const void *fun, int, size_t) {
     *n = on_occupancy(names()[fun].c_str());
     return cudaSuccess;

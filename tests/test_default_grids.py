@@ -42,6 +42,27 @@ int main(int argc, char **argv) {
 }
 """
 
+MSBFS = PROGRAM % "msbfs" + r"""
+#include <cstring>
+#include <sys/mman.h>
+extern "C" void on_launch(const char *name, void **args) {
+    if (strstr(name, "ms_persistent")) printf("%u\n", ((g5::MsArgs *)args[0])->nblocks);
+}
+// argv: vertices and CSR entries of a graph, ...  Prints the grid that a
+// search of each is launched with.
+int main(int argc, char **argv) {
+    for (int i = 1; i + 1 < argc; i += 2) {
+        const uint64_t n = atoll(argv[i]), e = atoll(argv[i + 1]), root = 0;
+        uint64_t need = 0;
+        if (g5_msbfs_workspace_size(n, e, 0, &need)) return 1;
+        void *work = mmap(nullptr, need, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS | MAP_NORESERVE, -1, 0);
+        if (work == MAP_FAILED || g5_msbfs_run(n, e, 0, &root, 1, work, need, nullptr, nullptr, nullptr)) return 2;
+        munmap(work, need);
+    }
+    return 0;
+}
+"""
+
 
 @pytest.fixture(scope="module")
 def bfs(tmp_path_factory):
@@ -53,3 +74,17 @@ def test_bfs_grid_by_vertices(bfs):
             1_300_000: 296, 2_000_000: 296, 3_000_000: 366, 4_194_304: 512, 1 << 25: 592, 1 << 31: 592}
     out = subprocess.run([bfs, *map(str, want)], check=True, capture_output=True, text=True).stdout
     assert [int(x) for x in out.split()] == list(want.values())
+
+
+@pytest.fixture(scope="module")
+def msbfs(tmp_path_factory):
+    return fake_cuda.build(tmp_path_factory.mktemp("msbfs_grid"), MSBFS)
+
+
+def test_batched_bfs_grid_by_entries(msbfs):
+    want = [(2, 2, 148), (260_000, 33_280_000, 148), (600_000, 9_600_000, 148), (400_000, 51_200_000, 296),
+            (1_000_000, 64_000_000, 296), (600_000, 76_800_000, 444), (1_000_000, 128_000_000, 592),
+            (1 << 22, 1 << 27, 592)]
+    out = subprocess.run([msbfs, *(str(x) for n, e, _ in want for x in (n, e))], check=True, capture_output=True,
+                         text=True).stdout
+    assert [int(x) for x in out.split()] == [b for _, _, b in want]
