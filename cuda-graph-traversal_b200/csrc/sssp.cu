@@ -64,8 +64,7 @@ constexpr int SSSP_TRACE = 256;      // phases recorded in the control block
 // expanded-set lists.  A warp's relaxation steps form a chain of dependent
 // round trips, so the chunk bounds the longest warp of a phase.  A multiple
 // of 32 x SSSP_EDGES (the entries a warp step covers).
-constexpr unsigned SSSP_CHUNK = 128;
-constexpr unsigned SSSP_TILE_SMALL = 64;  // for graphs of up to 2^22 vertices (sssp_tile)
+constexpr unsigned SSSP_CHUNK = 256;  // smaller on smaller graphs (sssp_tile)
 constexpr unsigned SSSP_GRAB = 32;
 // Sub-buckets: once a bucket's light frontier holds SPLIT_MIN light entries,
 // the rest of the bucket is processed in SUB equal sub-buckets in order
@@ -1924,8 +1923,16 @@ static int sssp_blocks(uint64_t nverts, int max_blocks) {
 // are a chain of dependent round trips that bounds a short phase, while on
 // large graphs the lookups of many small chunks cost more than they shorten
 // (64, 128 and 256: 16 K vertices 802, 865 and 915 us, 600 K 1641, 1797 and
-// 2059, 2.1 M 2919, 2948 and 3116, 16.8 M 9610, 8933 and 8972).
-static unsigned sssp_tile(uint64_t nverts) { return nverts <= (1ull << 22) ? SSSP_TILE_SMALL : SSSP_CHUNK; }
+// 2059, 2.1 M 2919, 2948 and 3116, 16.8 M 9.1, 8.4 and 8.5 ms, 34 M 15.5, 13.9 and
+// 13.6, 2000 packed graphs with 123 M 194, 151 and 138).  Rows that are not split
+// (a bucket wider than their light part) are read whole in every phase, twice
+// the chunks for the same relaxations: width 0.2, 64, 128 and 256: 600 K vertices
+// 2.4, 1.9 and 1.8 ms, 2 M 7.3, 6.3 and 5.5, 8.4 M 19.5, 14.2 and 10.9.
+static unsigned sssp_tile(uint64_t nverts, bool split_rows) {
+    return !split_rows || nverts > (1ull << 24) ? SSSP_CHUNK
+         : nverts > (1ull << 22)                ? SSSP_CHUNK / 2
+                                                : SSSP_CHUNK / 4;
+}
 
 }  // namespace g5
 
@@ -2102,8 +2109,8 @@ static int sssp_launch(const uint64_t *d_rowstarts, const int32_t *d_col, const 
     // opens, asks for buckets to the end.
     a.finish = p.pull == 0.0f && p.sub_min == 0 && !p.check_opens;
     a.refuse = (double)p.delta * RING * (1.0 + 1e-5);
-    a.big_deg = p.big_deg ? (unsigned)p.big_deg : sssp_tile(nverts);
-    a.chunk = p.chunk ? (unsigned)p.chunk : sssp_tile(nverts);
+    a.big_deg = p.big_deg ? (unsigned)p.big_deg : sssp_tile(nverts, split);
+    a.chunk = p.chunk ? (unsigned)p.chunk : sssp_tile(nverts, split);
     a.perm = p.perm;
     a.inv = p.inv;
     if (p.small && !d_roots) {

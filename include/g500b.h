@@ -433,7 +433,8 @@ typedef struct g5_sssp_params {
                        a test aid, same results; 0 = plain stores (default) */
     int32_t big_deg; /* list entries with more edges to expand are cut into
                        chunks across the grid; 0 = by the graph's size (64
-                       up to 2^22 vertices, else 128)                       */
+                       up to 2^22 vertices, 128 up to 2^24, else 256; 256
+                       where rows are not split at light_delta)             */
     int32_t chunk;   /* edges per chunk, a multiple of 64 up to 65536; 0 =
                        likewise.  Neither tile changes a result             */
     const uint32_t *perm; /* renumbered search (both set, from

@@ -1,5 +1,5 @@
-"""The default grids of the searches, by the graph's size (a fake CUDA runtime,
-fake_cuda.py, with four blocks an SM on 148 SMs)."""
+"""The default grids and list tiles of the searches, by the graph's size (a fake
+CUDA runtime, fake_cuda.py, with four blocks an SM on 148 SMs)."""
 from __future__ import annotations
 
 import subprocess
@@ -63,6 +63,34 @@ int main(int argc, char **argv) {
 }
 """
 
+SSSP = PROGRAM % "sssp" + r"""
+#include <cstring>
+#include <sys/mman.h>
+extern "C" void on_launch(const char *name, void **args) {
+    const g5::SsspArgs &a = *(g5::SsspArgs *)args[0];
+    if (strstr(name, "sssp_persistent")) printf("%u %u\n", a.big_deg, a.chunk);
+}
+// argv: vertices, bucket width (rows split at 0.1) ...  Prints the tiles that
+// a search of each is launched with.
+int main(int argc, char **argv) {
+    static uint64_t some[4];
+    for (int i = 1; i + 1 < argc; i += 2) {
+        const uint64_t n = atoll(argv[i]);
+        uint64_t need = 0;
+        if (g5_sssp_workspace_size(n, &need)) return 1;
+        void *work = mmap(nullptr, need, PROT_READ | PROT_WRITE, MAP_PRIVATE | MAP_ANONYMOUS | MAP_NORESERVE, -1, 0);
+        g5_sssp_params p = {};
+        p.delta = (float)atof(argv[i + 1]);
+        if (work == MAP_FAILED ||
+            g5_sssp_traverse(some, (int32_t *)some, (float *)some, (uint32_t *)some, 0.1f, n, 0, (float *)some,
+                             (int64_t *)some, work, need, &p, nullptr))
+            return 2;
+        munmap(work, need);
+    }
+    return 0;
+}
+"""
+
 
 @pytest.fixture(scope="module")
 def bfs(tmp_path_factory):
@@ -88,3 +116,16 @@ def test_batched_bfs_grid_by_entries(msbfs):
     out = subprocess.run([msbfs, *(str(x) for n, e, _ in want for x in (n, e))], check=True, capture_output=True,
                          text=True).stdout
     assert [int(x) for x in out.split()] == [b for _, _, b in want]
+
+
+@pytest.fixture(scope="module")
+def sssp(tmp_path_factory):
+    return fake_cuda.build(tmp_path_factory.mktemp("sssp_tiles"), SSSP)
+
+
+def test_sssp_tiles_by_vertices_and_rows(sssp):
+    want = [(2000, 0.1, 64), (1 << 22, 0.1, 64), ((1 << 22) + 1, 0.1, 128), (1 << 24, 0.05, 128),
+            ((1 << 24) + 1, 0.1, 256), (2000, 0.2, 256), (1 << 22, 0.11, 256), (1 << 25, 0.4, 256)]
+    out = subprocess.run([sssp, *(str(x) for n, d, _ in want for x in (n, d))], check=True, capture_output=True,
+                         text=True).stdout
+    assert [int(x) for x in out.split()] == [t for _, _, t in want for _ in range(2)]
