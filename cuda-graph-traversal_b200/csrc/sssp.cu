@@ -109,7 +109,14 @@ constexpr unsigned long long SPLIT_MIN = 1ull << 22, SPLIT_MIN_FEW = 1ull << 25;
 // 0.56; 200 K, 2^22.6, 0.75 and 0.69).  A kernel of its own because the
 // bucketed one is as large as it should get: with this loop inside, it
 // spilled three times as much.
+//
+// Searches from many sources on 2^30 entries and more stay in buckets: their
+// graphs' hubs are not in one bucket, so with half of the entries left many
+// hubs are still ahead, and the run without buckets relaxes their rows over
+// and over (300 graphs with 0.5 G entries 22.1 ms with the finish and 24.1 without, 800
+// with 1.4 G 66.9 and 62.5, 2000 with 3.9 G 169 and 148).
 constexpr unsigned long long FINISH_ENTRIES = 1ull << 22;
+constexpr unsigned long long FINISH_MULTI_BELOW = 1ull << 30;
 constexpr int FINISH_SHIFT = 1;
 constexpr float SSSP_PULL_RATIO = 1.0f;  // default heavy-phase pull threshold
 constexpr double PULL_WALK = 0.25;       // cost of a pull's bitmap walk, in CSR entries per vertex
@@ -252,6 +259,7 @@ struct SsspArgs {
     unsigned big_deg;  // list entries with more edges to expand go to the chunked big part
     unsigned chunk;    // edges of a big entry per warp grab
     bool finish;       // sssp_finish_kernel ends the search (and writes the outputs)
+    unsigned long long finish_below;  // it takes over only on graphs of fewer entries
     double refuse;     // a parent edge this long is beyond the bucket ring
     // Renumbered search (both set) or not (both nullptr): the CSR is in the
     // search's numbering, roots and outputs in the caller's; perm maps a
@@ -1149,7 +1157,8 @@ __global__ void __launch_bounds__(SSSP_THREADS, SSSP_MIN_BLOCKS) sssp_persistent
             bool ok = a.td != nullptr;
             for (int j = 0; j < SUB && ok; ++j) ok = __fadd_rn(s_sub[j], a.tiny) >= s_sub[j + 1];
             s_tiny_ok = ok;
-            s_stop = a.finish && e_total - settled_entries <= max(FINISH_ENTRIES, e_total >> FINISH_SHIFT);
+            s_stop = a.finish && e_total < a.finish_below &&
+                     e_total - settled_entries <= max(FINISH_ENTRIES, e_total >> FINISH_SHIFT);
         }
         __syncthreads();
         // Little left (every block sees the same counts): sssp_finish_kernel
@@ -1698,7 +1707,7 @@ __global__ void __launch_bounds__(SSSP_THREADS, 3) sssp_finish_kernel(SsspArgs a
             (double)pack_dist(p) - (double)pack_dist(__ldcg(&a.pack[(unsigned)p])) >= a.refuse)
             atomicOr(&c->error, DEVERR_RING);
     }
-    if (gtid == 0) {
+    if (gtid == 0 && round > 1) {  // the buckets left something
         c->buckets += 1;
         c->phases = pid0 + round;
     }
@@ -2108,6 +2117,7 @@ static int sssp_launch(const uint64_t *d_rowstarts, const int32_t *d_col, const 
     // Asking for pulls or sub-buckets by their thresholds, or for checked
     // opens, asks for buckets to the end.
     a.finish = p.pull == 0.0f && p.sub_min == 0 && !p.check_opens;
+    a.finish_below = d_roots ? FINISH_MULTI_BELOW : ~0ull;
     a.refuse = (double)p.delta * RING * (1.0 + 1e-5);
     a.big_deg = p.big_deg ? (unsigned)p.big_deg : sssp_tile(nverts, split);
     a.chunk = p.chunk ? (unsigned)p.chunk : sssp_tile(nverts, split);
