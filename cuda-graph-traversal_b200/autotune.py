@@ -70,11 +70,19 @@ def _descend(time_of, base: dict, axes: dict) -> tuple[float, dict, int]:
     return best_ms, best, count
 
 
-BFS_TILES = {"chunk": (128, 256, 512, 1024), "big_deg": (256, 1024, 4096), "lane_entries": (4, 8, 16, 32)}
-SSSP_TILES = {"chunk": (128, 256, 512, 1024), "big_deg": (64, 128, 256, 512)}
-# Where the descent over the tiles starts.
+# 0 is the library's default for the graph's size.
+BFS_TILES = {"chunk": (0, 128, 256, 512, 1024), "big_deg": (0, 256, 1024, 4096), "lane_entries": (0, 4, 8, 16, 32)}
+SSSP_TILES = {"chunk": (0, 64, 128, 256, 512, 1024), "big_deg": (0, 64, 128, 256, 512)}
+# Where the descent over axes without a 0 starts.
 BFS_DEFAULT_TILES = {"big_deg": 1024, "chunk": 256, "lane_entries": 8}
 SSSP_DEFAULT_TILES = {"big_deg": 256, "chunk": 256}
+
+
+def _first_tiles(axes: dict, otherwise: dict) -> dict:
+    """The tiles the descent over `axes` starts from: the library's defaults
+    (0) where an axis has them, which the table was timed with, so that a
+    tuned search is never one that lost to the untuned one."""
+    return {k: 0 if 0 in values else otherwise[k] for k, values in axes.items()}
 
 
 def tune_bfs(g: OnedGraph, roots, alphas=(6.0, 10.0, 14.0, 20.0, 28.0), betas=(12.0, 24.0, 48.0), grids=None,
@@ -83,7 +91,7 @@ def tune_bfs(g: OnedGraph, roots, alphas=(6.0, 10.0, 14.0, 20.0, 28.0), betas=(1
     search each) or a device tensor (one multi-root search, as on packed
     graphs); then, with those fixed, the work tiles of g5_bfs_params
     (big_deg, chunk, lane_entries) by coordinate descent over `tiles`
-    (None: the library's defaults)."""
+    (0 among an axis' values, and None for all: the library's defaults)."""
     bfs = BfsState(g)
     grids = _grids("bfs", g.nglobalverts) if grids is None else list(grids)
 
@@ -106,7 +114,7 @@ def tune_bfs(g: OnedGraph, roots, alphas=(6.0, 10.0, 14.0, 20.0, 28.0), betas=(1
     out = {"alpha": best[1], "beta": best[2], "blocks": best[3], "big_deg": 0, "chunk": 0, "lane_entries": 0}
     ms, count = best[0], len(table)
     if tiles:
-        out.update(**BFS_DEFAULT_TILES)
+        out.update(_first_tiles(tiles, BFS_DEFAULT_TILES))
         ms, out, more = _descend(time_of, out, tiles)
         count += more
     return {"kind": "bfs", **out, "ms": round(ms, 4), "candidates": count}
@@ -117,8 +125,9 @@ def tune_sssp(g: OnedGraph, roots, deltas=(0.08, 0.1, 0.2, 0.4), grids=None, pul
     """Best (delta, blocks, pull, sub_min) for SSSP over `roots` (a list: one
     search each; a device tensor: one multi-source search).  pull / sub_min
     are g5_sssp_params' heavy-phase pull threshold and sub-bucket threshold
-    (0 = the library's default, -1 = off).  Then the list tiles (big_deg,
-    chunk) by coordinate descent over `tiles`."""
+    (0 = the library's default, -1 = off; the search's finish runs only where
+    both are 0).  Then the list tiles (big_deg, chunk) by coordinate descent
+    over `tiles`, as in tune_bfs."""
     st = SsspState(g)
     grids = _grids("sssp", g.nglobalverts) if grids is None else list(grids)
 
@@ -142,7 +151,7 @@ def tune_sssp(g: OnedGraph, roots, deltas=(0.08, 0.1, 0.2, 0.4), grids=None, pul
     out = {"delta": best[1], "blocks": best[2], "pull": best[3], "sub_min": best[4], "big_deg": 0, "chunk": 0}
     ms, count = best[0], len(table)
     if tiles:
-        out.update(**SSSP_DEFAULT_TILES)
+        out.update(_first_tiles(tiles, SSSP_DEFAULT_TILES))
         ms, out, more = _descend(time_of, out, tiles)
         count += more
     return {"kind": "sssp", **out, "ms": round(ms, 4), "candidates": count}
