@@ -874,7 +874,9 @@ __device__ __forceinline__ uint64_t byte_mask_of_bits(unsigned s8) {
 // (32 roots) of vertices 4q..4q+3 into 32 stores of 4 bytes, one per root, a
 // warp's stores covering 128 consecutive bytes of one root's output.  The
 // bit planes become depth bytes by byte permutes and 8x8 bit transposes
-// (about 7 instructions per output byte).  Every row is read once.
+// (about 7 instructions per output byte).  Every row is read once.  Four
+// blocks an SM, which spill 16 bytes a thread: 256 roots on 4.2 M vertices 0.72
+// ms, two 0.81.
 constexpr int EX_V = 128;
 static_assert(EX_V == 4 * 32, "a warp's 32 threads take the 128 vertices four each");
 
@@ -972,19 +974,22 @@ __global__ void __launch_bounds__(256, 4) ms_export_u8_kernel(const unsigned *__
     }
 }
 
-// Blocks of a batch by default: one an SM (a quarter of what fits) up to 2^25
-// CSR entries, two up to 2^26, three up to 3 x 2^25, then all that fit; where
-// levels are short, more blocks only crowd the cursors and the barrier.  256
-// roots on 148, 296, 444 and 592 blocks: 260 K vertices and 8 M entries 1.14, 1.34, 1.43
-// and 1.53 ms, 600 K and 19 M 1.64, 1.76, 1.86 and 2.06, 400 K and 51 M 1.69, 1.45, 1.54 and
-// 1.65, 600 K and 77 M 2.39, 2.04, 1.90 and 2.02, 1 M and 128 M 3.25, 2.39, 2.35 and 2.28.
-// (By vertices, as the BFS's grid, dense graphs got too few.)
-static int ms_blocks(uint64_t nentries, int max_blocks) {
+// Blocks of a batch by default, by its work (entries, and the passes over the
+// vertices as 8 entries each): one an SM (a quarter of what fits) up to 46 M,
+// two up to 101 M, three up to 134 M, then all that fit; where levels are short,
+// more blocks only crowd the cursors and the barrier.  256 roots on 148, 296,
+// 444 and 592 blocks: 260 K vertices and 8 M entries (10 M) 1.14, 1.34, 1.43 and 1.53
+// ms, 1 M and 32 M (40 M) 1.64, 1.79, 1.88 and 2.01, 4 M and 16 M (48 M) 2.43, 2.13, 2.25
+// and 2.28, 400 K and 51 M (54 M) 1.69, 1.45, 1.54 and 1.65, 4 M and 64 M (96 M) 3.49, 2.30,
+// 2.41 and 2.47, 8 M and 64 M (128 M) 5.08, 3.28, 2.87 and 2.92, 1 M and 128 M (136 M) 3.25,
+// 2.39, 2.35 and 2.28.
+static int ms_blocks(uint64_t nverts, uint64_t nentries, int max_blocks) {
     const int sm = std::max(1, max_blocks / 4);
-    return nentries <= (1ull << 25) ? sm
-         : nentries <= (1ull << 26) ? 2 * sm
-         : nentries <= (3ull << 25) ? 3 * sm
-                                    : max_blocks;
+    const uint64_t work = nentries + 8 * nverts;
+    return work <= (11ull << 22) ? sm
+         : work <= (3ull << 25)  ? 2 * sm
+         : work <= (1ull << 27)  ? 3 * sm
+                                 : max_blocks;
 }
 
 static int ms_max_blocks(int *out) {
@@ -1079,7 +1084,7 @@ extern "C" int g5_msbfs_run(uint64_t nverts, uint64_t nentries, int depth_bits, 
                  "g5_msbfs_run: bad params");
     int max_blocks = 0;
     if ((rc = ms_max_blocks(&max_blocks))) return rc;
-    const int blocks = p.blocks > 0 ? std::min(p.blocks, max_blocks) : ms_blocks(nentries, max_blocks);
+    const int blocks = p.blocks > 0 ? std::min(p.blocks, max_blocks) : ms_blocks(nverts, nentries, max_blocks);
     cudaStream_t st = (cudaStream_t)stream;
     DeviceInfo di;
     if ((rc = device_info(&di))) return rc;

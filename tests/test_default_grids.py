@@ -109,10 +109,10 @@ def msbfs(tmp_path_factory):
     return fake_cuda.build(tmp_path_factory.mktemp("msbfs_grid"), MSBFS)
 
 
-def test_batched_bfs_grid_by_entries(msbfs):
-    want = [(2, 2, 148), (260_000, 33_280_000, 148), (600_000, 9_600_000, 148), (400_000, 51_200_000, 296),
-            (1_000_000, 64_000_000, 296), (600_000, 76_800_000, 444), (1_000_000, 128_000_000, 592),
-            (1 << 22, 1 << 27, 592)]
+def test_batched_bfs_grid_by_entries_and_vertices(msbfs):
+    want = [(2, 2, 148), (260_000, 33_280_000, 148), (600_000, 9_600_000, 148), (1_000_000, 32_000_000, 148),
+            (4_000_000, 16_000_000, 296), (400_000, 51_200_000, 296), (4_000_000, 64_000_000, 296),
+            (8_000_000, 64_000_000, 444), (1_000_000, 128_000_000, 592), (1 << 22, 1 << 27, 592)]
     out = subprocess.run([msbfs, *(str(x) for n, e, _ in want for x in (n, e))], check=True, capture_output=True,
                          text=True).stdout
     assert [int(x) for x in out.split()] == [b for _, _, b in want]
