@@ -55,12 +55,12 @@ constexpr unsigned STAGE_D = 32;     //                   the sub-bucket's expan
 static_assert(STAGE_F >= 32 && STAGE_S >= 32, "staging slices hold one warp step");
 static_assert(STAGE_R <= 32 && STAGE_Q <= 32, "stage_push writes a full slice with one lane per entry");
 constexpr int SSSP_TRACE = 256;      // phases recorded in the control block
-// List entries with more edges to expand than this go to the big part (cut
-// into SSSP_CHUNK chunks across the grid), and a warp grabs at most SSSP_GRAB
+// List entries with more edges to expand than the tile go to the big part (cut
+// into chunks of a tile across the grid), and a warp grabs at most SSSP_GRAB
 // small entries at once: a grab holds at most SSSP_GRAB times as many edges,
 // so no warp is left with a long tail of relaxations at the end of a phase.
-// SSSP_CHUNK is the default of both g5_sssp_params.big_deg and .chunk.
-// Chunk of a long row taken by one warp in the frontier, heavy-set and
+// SSSP_CHUNK is the largest default of g5_sssp_params.big_deg and .chunk: the
+// chunk of a long row taken by one warp in the frontier, heavy-set and
 // expanded-set lists.  A warp's relaxation steps form a chain of dependent
 // round trips, so the chunk bounds the longest warp of a phase.  A multiple
 // of 32 x SSSP_EDGES (the entries a warp step covers).
@@ -88,27 +88,31 @@ constexpr int SUB = 32;
 // first phases on, before most repeats are made.  Split at 2^22 against not
 // split: 8.4 M vertices and 268 M entries 5.9 and 6.6 ms, 6 M and 192 M 4.0 and
 // 4.6, 3 M and 192 M 3.8 and 4.2; 5 M and 160 M 4.5 and 4.3, 4.2 M and 134 M 4.2 and
-// 3.6, 2 M and 64 M 3.4 and 1.9, 1 M and 64 M 2.3 and 1.7.  Below SPLIT_ENTRIES
-// only a frontier of SPLIT_MIN_FEW splits.
+// 3.6, 2 M and 64 M 3.4 and 1.9, 1 M and 64 M 2.3 and 1.7.  On a part of the device
+// the repeats take longer and the windows do not, so there the line is at
+// SPLIT_BLOCK entries a block: 4.2 M and 134 M on 222 blocks 4.2 and 4.7 ms, on 55
+// 9.5 and 15.4, 2 M and 67 M on 148 3.5 and 3.3, on 111 4.1 and 4.2, on 55 6.5 and
+// 7.5, 1.5 M and 96 M on 222 3.3 and 2.8, on 148 3.7 and 3.7, on 111 4.2 and 4.8.  Below
+// the line only a frontier of SPLIT_MIN_FEW splits.
 // With many sources (packed graphs) a large frontier is many small ones, whose
 // vertices are seldom lowered again: 90 graphs with 167 M entries in all take
 // 13 ms unsplit and 18 split, so there the line is where it hardly matters.
 // Defaults; g5_sssp_params.sub_min overrides.
-constexpr unsigned long long SPLIT_ENTRIES = 5ull << 25;
+constexpr unsigned long long SPLIT_ENTRIES = 5ull << 25, SPLIT_BLOCK = 9ull << 16;
 constexpr unsigned long long SPLIT_MIN = 1ull << 22, SPLIT_MIN_FEW = 1ull << 25;
 // The bucketed kernel hands over to sssp_finish_kernel once the rows of the
 // vertices not settled hold at most FINISH_ENTRIES entries or 2^-FINISH_SHIFT
 // of all.  What is left after the bucket that holds the hubs hangs off settled
 // vertices and is seldom lowered twice, but it went through some 20 buckets
 // of at least three phases, about 10 us each however small: with the finish
-// 600 K vertices take 1.0 ms instead of 1.5, 90 packed graphs 7.8 instead of
-// 11.7 (8.7 when a quarter of the entries is the line instead of half).  A
+// 600 K vertices take 1.05 ms instead of 1.7, 90 packed graphs 7.9 instead of
+// 11.3 (a tenth longer when a quarter of the entries is the line, not half).  A
 // search handed over at once relaxes each entry about five times, which beats
-// the buckets' phases up to about 2^22 entries (16 K vertices 0.25 ms, in
-// buckets 0.67; 100 K vertices, 2^21.6 entries, 0.40 ms, in buckets first
-// 0.56; 200 K, 2^22.6, 0.75 and 0.69).  A kernel of its own because the
-// bucketed one is as large as it should get: with this loop inside, it
-// spilled three times as much.
+// the buckets' phases up to about 2^22 entries (16 K vertices 0.26 ms, in
+// buckets 0.84; 65 K, 2^21 entries, 0.41, in buckets first 0.49; 100 K, 2^21.6,
+// 0.46 and 0.53; 200 K, 2^22.6, 0.69 and 0.68).  A kernel of its own: with this
+// loop inside, the bucketed one spilled three times as much, and builds of
+// that form hung on a star graph for a cause that was never found.
 //
 // Searches from many sources on 2^30 entries and more stay in buckets: their
 // graphs' hubs are not in one bucket, so with half of the entries left many
@@ -2089,7 +2093,7 @@ static int sssp_launch(const uint64_t *d_rowstarts, const int32_t *d_col, const 
     a.delta = p.delta;
     a.pull_ratio = p.pull == 0.0f ? SSSP_PULL_RATIO : p.pull;
     a.split_min = p.sub_min == 0 ? (d_roots ? SPLIT_MIN_FEW : SPLIT_MIN) : p.sub_min < 0 ? ~0ull : (unsigned long long)p.sub_min;
-    a.split_entries = p.sub_min == 0 ? SPLIT_ENTRIES : 0;
+    a.split_entries = p.sub_min == 0 ? std::min(SPLIT_ENTRIES, (unsigned long long)blocks * SPLIT_BLOCK) : 0;
     a.pack = w.pack;
     a.fstamp = w.fstamp;
     a.sstamp = w.sstamp;
@@ -2114,8 +2118,8 @@ static int sssp_launch(const uint64_t *d_rowstarts, const int32_t *d_col, const 
     a.nblocks = (unsigned)blocks;
     a.limit_ns = wait_limit_ns();
     a.check_opens = p.check_opens != 0;
-    // Asking for pulls or sub-buckets by their thresholds, or for checked
-    // opens, asks for buckets to the end.
+    // Asking for pulls or sub-buckets by their thresholds (the defaults' values
+    // too), or for checked opens, asks for buckets to the end.
     a.finish = p.pull == 0.0f && p.sub_min == 0 && !p.check_opens;
     a.finish_below = d_roots ? FINISH_MULTI_BELOW : ~0ull;
     a.refuse = (double)p.delta * RING * (1.0 + 1e-5);
