@@ -637,8 +637,8 @@ def run_sssp_batched(G, dev, scale, ef, nsources=32, reps=3):
             "entries_scanned_per_entry": round(st.entries_scanned / max(1, g.nlocaledges), 2),
             "setup_s": round(time.time() - t0, 2),
             "timing": "device events, min of 3 after one warm-up; plain = single-source traverse, reset untimed",
-            "note": "a win up to about 2^20 vertices (SCALE 14: 10-13x, 18: 3.6-3.9x, 20: 1.5-1.7x); from SCALE 22 "
-                    "the single-source delta-stepping search is faster (0.7x at 22, 0.27x at 26)"}
+            "note": "against 32 single searches, resets timed: SCALE 14 7.6x, 16 6.2x, 18 2.7x, 20 1.1x, 21 0.9x, "
+                    "22 0.7x; from SCALE 21 the single-source search is faster"}
 
 
 def run_packed(G, dev, ngraphs, smin, smax, ef, reps=3):

@@ -1137,6 +1137,8 @@ def oned_graph_sssp_run(g: OnedGraph, sssp: SsspState, root: int, delta: float =
                         pull: float = 0.0, sub_min: int = 0, small: bool | None = None, stream=None,
                         check_opens: bool = False, big_deg: int = 0, chunk: int = 0) -> None:
     """oned_graph_sssp_run (src/traversal.h:52), delta 0.1 as the reference.
+    pull / sub_min: g5_sssp_params' thresholds (0 = defaults, which leave the
+    search's end to the finish; any other value asks for buckets to the end).
     check_opens: the bucket and sub-bucket opens exchange their stamps and
     fail the search if a queue held a vertex twice (a test aid).  big_deg /
     chunk: the work tiles of g5_sssp_params (0 = defaults)."""
@@ -1149,7 +1151,7 @@ def oned_graph_sssp_run(g: OnedGraph, sssp: SsspState, root: int, delta: float =
 
 
 def sssp_multi_workspace(g: OnedGraph) -> torch.Tensor:
-    """Scratch of oned_graph_sssp_multi (about 276 bytes per vertex)."""
+    """Scratch of oned_graph_sssp_multi (about 288 bytes per vertex)."""
     nb = C.c_uint64()
     _check(lib.g5_sssp_multi_workspace_size(g.nglobalverts, C.byref(nb)))
     return _workspace(nb.value, g.device)
@@ -1181,8 +1183,8 @@ def oned_graph_sssp_multi(g: OnedGraph, sources, work: torch.Tensor | None = Non
     dist[s] / pred[s] equal oned_graph_sssp_run's outputs from sources[s]
     bit for bit (float32 distances, -1.0 / -1 where unreached).  Runs on the
     graph's renumbered SSSP copy when it has one (sources and outputs stay
-    in the caller's numbering).  delta: the shared bucket width (0 = 0.1;
-    results never depend on it).  `work`: sssp_multi_workspace(g), else one
+    in the caller's numbering).  delta: the shared bucket width (0 = no
+    buckets, the fast setting; results never depend on it).  `work`: sssp_multi_workspace(g), else one
     is allocated; `dist` / `pred`: [len(sources), N] outputs to reuse.
     sync=False: no wait (statistics None; sssp_multi_status reads them)."""
     src = [int(x) for x in sources]

@@ -50,7 +50,10 @@ constexpr int BFS_THREADS = 256;
 // 36 rows with 64 K edges) 128 / 256 takes 95 us, 256 / 256 103 and 256 / 1024
 // 139.  In a wide top-down level the chunks' one cursor is the bound instead:
 // 37 M edges on 34 M vertices take 1.04 ms with 128 / 256 and 0.69 with 256 /
-// 1024, the defaults from BFS_TILE_VERTICES on.
+// 1024, the defaults from BFS_TILE_VERTICES on.  Whole searches, fine against
+// coarse: 2 M vertices 180 and 209 us, 4.2 M 213 and 285, 6 M 545 and 454 on
+// one graph and 281 and 312 on another, 8.4 M 385 and 390 (mean of four), 16.8 M
+// 519 and 520, 34 M 862 and 856.
 constexpr unsigned BFS_CHUNK = 128, BFS_CHUNK_LARGE = 256;
 constexpr unsigned BFS_BIG_DEG = 256, BFS_BIG_DEG_LARGE = 1024;
 constexpr uint64_t BFS_TILE_VERTICES = 1ull << 22;

@@ -7,7 +7,7 @@
 // for all its sources reads and lowers one 256-byte row with atomicMin: the
 // edge's column entry and weight are loaded once for 32 searches.  Work goes
 // in distance order, as in delta-stepping, on one bucket index for all
-// sources: a vertex whose word for some source dropped has that source's bit
+// sources (without a bucket width everything is in bucket 0): a vertex whose word for some source dropped has that source's bit
 // set in its change mask and its smallest pending bucket (floor(dist /
 // delta)) in vbkt; the first bit set since the vertex was last taken queues
 // it.  A round of bucket b takes each queued vertex whose vbkt <= b (its mask
@@ -34,9 +34,8 @@ constexpr int MSS_THREADS = 256;
 constexpr int MSS_SOURCES = 32;    // one warp lane per source
 // Longer rows are cut into chunks of this many entries: one warp step, whose
 // round trips (eight entries at a time) are then the longest chain of a round.
-// 32 sources on 4 K, 33 K and 131 K vertices: 0.51, 1.30 and 4.29 ms, with 64
-// 0.71, 1.48 and 4.30, with 256 (and a binary search per chunk) 1.42, 2.52 and
-// 5.54.
+// 32 sources on 4 K, 33 K and 131 K vertices: 0.50, 1.32 and 4.15 ms, with 64
+// 0.69, 1.47 and 4.10, with 256 1.40, 2.46 and 5.14.
 constexpr unsigned MSS_CHUNK = 32;
 constexpr unsigned long long MSS_NONE = ~0ull;
 constexpr int MSS_MAX_ROUNDS = 1 << 20;
@@ -142,8 +141,10 @@ __device__ __forceinline__ void mss_note(const MssArgs &a, unsigned v, unsigned 
 
 // Entries of a row whose targets' words are loaded together: relaxing one
 // entry is a chain of a load and an atomic (about 1 us), and a warp that took
-// its entries one by one spent all its time in it.  32 sources on 130 K
-// vertices: 6.7 ms one by one, 5.9 by fours, 4.9 by eights; sixteen spill.
+// its entries one by one spent all its time in it.  32 sources on 4 K, 33 K and
+// 131 K vertices: 0.50, 1.32 and 4.15 ms by eights, 0.59, 1.39 and 4.12 by fours,
+// 0.58, 1.58 and 5.05 one by one; sixteen do not fit the registers (0.64, 2.16
+// and 7.84), eight spill 32 bytes a thread.
 constexpr int MSS_BATCH = 8;
 
 // Relaxes entries [b, e) of u's row for the sources in mask m (lane s =

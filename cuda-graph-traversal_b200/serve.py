@@ -16,10 +16,12 @@ free it launches the oldest waiting work:
 * pending SSSP queries of a graph of at most `sssp_batch_max_vertices`
   (2^20) vertices, when at least `sssp_batch_min` (2) wait, become one
   batched search of up to 32 sources (g5_sssp_multi_run) on that graph's
-  batched-SSSP workspace, which answers 32 sources 1.5-13x faster than 32
-  single searches on graphs of 2^20 down to 2^14 vertices; otherwise (and on
-  larger graphs, where the single search is the faster one) an SSSP query
-  runs on its own on a pooled SSSP workspace of that graph.
+  batched-SSSP workspace, which answers 32 sources 7.6x faster than 32 single
+  searches with the device to themselves on graphs of 2^14 vertices, 6.2x on
+  2^16, 2.7x on 2^18 and 1.1x on 2^20 (8 sources 2.4x, 2.0x, 1.0x and 0.4x; 2
+  sources 0.7x and less); otherwise (and on larger graphs, where the single
+  search is the faster one) an SSSP query runs on its own on a pooled SSSP
+  workspace of that graph.
 
 Every search is a persistent cooperative kernel whose grid is sized to its
 graph (g5_*_grid); launches run concurrently only while the sum of their

@@ -399,7 +399,8 @@ int g5_bfs_run_static(const uint64_t *d_rowstarts, const int32_t *d_col, uint64_
  * d_dist[v] = -1 where pred is -1, 0 at the root, the tree depth where the
  * parent chain reaches the root through CSR edges, INT64_MAX otherwise.
  * d_work needs g5_validate_workspace_size bytes (not the BFS workspace,
- * whose statistics it would overwrite).  Synchronises once per level. */
+ * whose statistics it would overwrite).  Synchronises once per 64 levels of
+ * the tree. */
 int g5_bfs_dist_from_pred(const uint64_t *d_rowstarts, const int32_t *d_col, uint64_t nverts,
                           const int64_t *d_pred, uint64_t root, int64_t *d_dist, void *d_work,
                           uint64_t work_bytes, void *stream);
@@ -413,12 +414,17 @@ typedef struct g5_sssp_params {
     float pull;     /* a bucket's heavy phase pulls (each unsettled vertex scans
                        its own heavy entries) when the bucket's rows hold at
                        least pull x the entries of all unsettled vertices'
-                       rows; 0 = default (1.0), < 0 = always push           */
+                       rows; 0 = default (1.0), < 0 = always push.  A
+                       search with this and sub_min 0 and check_opens 0
+                       leaves its end to the finish (see g5_sssp_run); any
+                       other value, the defaults' own too, asks for buckets
+                       to the end                                            */
     int32_t sub_min; /* once a bucket's light frontier holds this many light
                        CSR entries, the rest of the bucket runs in 32
                        sub-buckets in distance order; 0 = default (2^22 on
-                       graphs of 5 x 2^25 CSR entries and more, 2^25 on
-                       smaller ones and with several sources), < 0 = never  */
+                       graphs of 5 x 2^25 CSR entries and more, or 9 x 2^16
+                       a block of a smaller grid; 2^25 on smaller ones and
+                       with several sources), < 0 = never                   */
     int32_t small;   /* 1: the source's component is small (outside the main
                        component): one lean block, label-correcting rounds,
                        same distances and parents; 0 = the bucketed search  */
@@ -456,8 +462,18 @@ int g5_sssp_workspace_size(uint64_t nverts, uint64_t *bytes);
  * than `light_delta` as produced by g5_csr_fill; it is used when
  * params->delta <= light_delta (light edges are then those below
  * light_delta), otherwise rows are filtered by weight against delta.
- * The bucket ring holds 31 buckets ahead, so delta must exceed
- * (largest weight) / 30 (G5_ERR_INVALID from the search otherwise). */
+ * Once the rows of the vertices not settled yet hold at most 2^22 entries or
+ * half of all, the search leaves the buckets: the finish relaxes whole rows
+ * until no distance drops.  Same distances and parents; graphs of up to 2^22
+ * entries are searched by it alone, searches from several sources on 2^30
+ * entries and more never, nor those that set params->pull, sub_min or
+ * check_opens.
+ * The bucket ring holds 31 buckets ahead, so delta must exceed (largest
+ * weight) / 30 for every search to be answered.  Otherwise an edge of 32 x
+ * delta and more on a shortest path fails the search (G5_ERR_INVALID from its
+ * status calls); a shorter edge beyond 30 x delta, and an edge that lowers a
+ * distance only for a time, fail it when a bucket meets them, while the
+ * finish, which has no ring, goes on. */
 int g5_sssp_run(const uint64_t *d_rowstarts, const int32_t *d_col, const float *d_w, const uint32_t *d_light_deg,
                 float light_delta, uint64_t nverts, uint64_t root, float *d_dist, int64_t *d_pred, void *d_work,
                 uint64_t work_bytes, const g5_sssp_params *params, void *stream);
@@ -469,7 +485,8 @@ int g5_sssp_run(const uint64_t *d_rowstarts, const int32_t *d_col, const float *
  * (distances, stamps, settled bitmap) and its control block and, when given
  * d_dist and d_pred (both or neither), fills them with -1.0f / -1;
  * g5_sssp_traverse (on a state reset since its last search) runs the
- * persistent kernel and writes d_dist / d_pred.
+ * persistent kernel and the finish's, two launches on `stream` with one grid,
+ * and writes d_dist / d_pred.
  * When the traverse gets the same output arrays the reset pre-filled, it
  * writes only the reached vertices (O(reached) work); otherwise it writes
  * all nverts entries. */
@@ -506,10 +523,12 @@ int g5_sssp_last_status(const void *d_work, uint64_t work_bytes, uint64_t *bucke
 /* Counters and per-phase trace of the last g5_sssp_run on this workspace
  * (synchronises): counts[7] = edges looked at, edges into settled vertices,
  * atomicMin issued, distances lowered, bucket-queue pushes, same-bucket
- * frontier and sub-bucket pushes, heavy phases run as pulls; per phase (up
- * to 256) its kind (0 bucket open, 1 light, 2 heavy push, 3 heavy pull,
- * 4 sub-bucket open, 5 bucket split into sub-buckets), input list size,
- * device milliseconds and edges looked at.  Any output pointer may be NULL. */
+ * frontier and sub-bucket pushes, heavy phases run as pulls (the finish adds
+ * to the first and the fourth only); per phase (up to 256) its kind (0 bucket
+ * open, 1 light, 2 heavy push, 3 heavy pull, 4 sub-bucket open, 5 bucket split
+ * into sub-buckets, 6 a sub-bucket's deferred edges, 7 a round of the finish),
+ * input list size, device milliseconds and edges looked at (0 for the
+ * finish's rounds).  Any output pointer may be NULL. */
 int g5_sssp_last_trace(const void *d_work, uint64_t work_bytes, uint64_t counts[7], int max_phases, int32_t *kind,
                        uint64_t *size, double *phase_ms, uint64_t *phase_edges, int32_t *nphases, void *stream);
 
@@ -573,7 +592,8 @@ typedef struct g5_msbfs_params {
     int mode;       /* 0 automatic, 1 top-down only, 2 pull only */
     int check_frontier; /* pull levels test the frontier bitmap before reading a neighbour's row:
                            0 when under half the entries lead into the frontier, 1 always, 2 never */
-    int blocks;     /* persistent grid (0 = every co-resident block) */
+    int blocks;     /* persistent grid; 0 = by the graph's entries and vertices, from one block an SM to
+                       every co-resident block */
 } g5_msbfs_params;
 
 typedef struct g5_msbfs_stats {
@@ -629,15 +649,15 @@ int g5_msbfs_last_trace(const void *d_work, uint64_t work_bytes, int max_levels,
  * reference runs one source at a time, src/traversal.cu:638-711): one warp
  * lane per source, each vertex's 32 packed (distance, parent) words side by
  * side, so an edge's column entry and weight are read once for every
- * source; label-correcting rounds over the vertices whose words dropped, in
- * buckets of width delta shared by the sources (0 = 0.1), as delta-stepping
- * takes them.
+ * source; label-correcting rounds over the vertices whose words dropped,
+ * all of them each round (delta 0, the fast setting) or in buckets of width
+ * delta shared by the sources, as delta-stepping takes them.
  * Distances and parents equal g5_sssp_run's for each source bit for bit.
  * Any row order of the CSR will do (the renumbered SSSP copy: pass its
  * perm / inv, sources and outputs stay in the caller's numbering).
  * d_dist / d_pred (optional, nsources x nverts, source-major: entry
  * s * nverts + v) receive -1.0f / -1 where unreached.  Synchronises when
- * h_stats is given.  Scratch: g5_sssp_multi_workspace_size (about 276 bytes
+ * h_stats is given.  Scratch: g5_sssp_multi_workspace_size (about 288 bytes
  * per vertex). */
 typedef struct g5_sssp_multi_stats {
     int32_t rounds;            /* relaxation rounds                                   */
@@ -658,9 +678,10 @@ int g5_sssp_multi_grid(uint64_t nverts, int32_t *blocks, int32_t *max_blocks);
 
 /* ------------------------------------------------------------- grids ----- */
 /* Grid (blocks) sized for a graph of nverts vertices -- what g5_bfs_* and
- * g5_sssp_* launch with params.blocks = 0 (g5_msbfs_run then takes every
- * co-resident block instead) -- and the most blocks of the kernel that fit
- * on the device at once.  A caller that runs searches on several streams at
+ * g5_sssp_* launch with params.blocks = 0 (g5_msbfs_run and
+ * g5_sssp_multi_run then take grids that are fastest with the device to
+ * themselves instead) -- and the most blocks of the kernel (of each of a
+ * search's kernels) that fit on the device at once.  A caller that runs searches on several streams at
  * the same time passes these grids in params.blocks and keeps their sum
  * within max_blocks, so every cooperative grid can be resident together. */
 int g5_bfs_grid(uint64_t nverts, int32_t *blocks, int32_t *max_blocks);
