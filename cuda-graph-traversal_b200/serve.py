@@ -175,7 +175,7 @@ class GraphServer:
         if g.nglobalverts > self.sssp_batch_max_vertices:
             return None
         if self.mss[gi] is None:
-            if not self._fits(404 * g.nglobalverts):  # workspace + 32 distance rows
+            if not self._fits(416 * g.nglobalverts):  # workspace + 32 distance rows
                 return None
             self.mss[gi] = SsspMultiState(g, SSSP_BATCH_MAX)
             self.stats.workspaces[f"sssp_multi{gi}"] = self.mss[gi].work.numel()
